@@ -66,6 +66,8 @@ struct PackedFactors {
 };
 size_t packed_factor_doubles(int M);
 void pack_line_factors(const LineFactors &f, std::vector<double> &out);
+// Factors of the same axis for solve_fast (solve_line.cu).
+void pack_fast_factors(const LineFactors &f, std::vector<double> &out);
 
 // ----------------------------------------------------------------- table
 }  // namespace eg
@@ -105,12 +107,14 @@ struct einspline_gb300_table {
   std::unordered_map<int, int> slot_of;
   void *staging = nullptr;          // device, cap * points * ncomp values of the input type
   int in_bytes = 4;                 // bytes per input real (4 for s/c, 8 for d/z)
-  double *work_a = nullptr;         // device FP64 [Mx][My][Mz][cap*ncomp]
+  double *work_a = nullptr;         // device FP64 [Mx][My][Mz][cap*ncomp] (fast_solve: [cap*ncomp])
   double *work_w = nullptr;         // device FP64 [Nx][Ny][Nz][cap*ncomp]
   float *colmax = nullptr;          // device, cap*ncomp
   int *slot_spline_d = nullptr;     // device, cap
   double *factors_d = nullptr;      // device, 3 packed factor sets
   size_t factor_off[3] = {0, 0, 0};
+  size_t fast_off[3] = {0, 0, 0};   // the same buffer: the factors of solve_fast
+  bool fast_solve = false;          // solved by solve_fast (fast_solve_fits)
   cudaStream_t stream = nullptr;
 
   // single-point entry scratch: 40 * ncol output reals in mapped pinned
@@ -177,6 +181,14 @@ int table_set(Table *t, int first, int count, const void *data, bool from_device
 int table_set_bc(Table *t, int spline, const void *data, int lcode, int rcode, const double lval[2],
                  const double rval[2]);
 int table_flush(Table *t);
+// The solve of 3D tables whose result is rounded to 32 or 16 bits
+// (solve_line.cu): the n queued splines' data in t->staging become t's FP32
+// columns, or for 16-bit storage the FP64 coefficients in t->work_w with the
+// columns' largest magnitudes in t->colmax.  A line has to fit in a block's
+// shared memory with 31 others.
+constexpr int kFastMaxLine = 288;
+bool fast_solve_fits(const Table *t);
+int solve_fast(Table *t, int n, cudaStream_t s);
 // Rebuilds the double-float shadow of an FP64 table when fp64_mode is 1 and
 // the table changed since it was made.
 int table_df_refresh(Table *t);

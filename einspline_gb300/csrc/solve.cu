@@ -358,6 +358,8 @@ __global__ void k_scales(int st, const unsigned int *colmax, int nslots, int nco
   }
 }
 
+constexpr int kStoreCells = 8;
+
 // Rounds one FP64 coefficient to the storage type at table[o].
 template <int ST>
 __device__ __forceinline__ void store_coef(void *table, int64_t o, double w, double inv) {
@@ -372,17 +374,26 @@ __device__ __forceinline__ void store_coef(void *table, int64_t o, double w, dou
   }
 }
 
+// A thread owns one column and walks the cells of its grid row, eight reads
+// in flight: its factor and table column are looked up once.  64^3 x 1024
+// F16: 1.15 ms (one element a thread: 1.41 ms), bound by the FP64 multiply
+// and conversion of each coefficient.
 template <int ST>
-__global__ void k_store(const double *__restrict__ W, int64_t ncells, int ncw, int ncomp,
-                        const int *__restrict__ slot_spline, const double *__restrict__ inv,
-                        void *__restrict__ table, int64_t zs) {
-  const int cblocks = (ncw + blockDim.x - 1) / blockDim.x;
-  const int64_t cell = blockIdx.x / cblocks;
-  const int c = (int)(blockIdx.x % cblocks) * blockDim.x + threadIdx.x;
-  if (cell >= ncells || c >= ncw) return;
-  const double w = W[cell * ncw + c];
+__global__ void __launch_bounds__(128) k_store(const double *__restrict__ W, int64_t ncells, int ncw, int ncomp,
+                                               const int *__restrict__ slot_spline, const double *__restrict__ inv,
+                                               void *__restrict__ table, int64_t zs) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ncw) return;
   const int64_t tcol = (int64_t)slot_spline[c / ncomp] * ncomp + (c % ncomp);
-  store_coef<ST>(table, cell * zs + tcol, w, is16(ST) ? inv[c] : 1.0);
+  const double iv = is16(ST) ? inv[c] : 1.0;
+  for (int64_t cell = (int64_t)blockIdx.y * kStoreCells; cell < ncells; cell += (int64_t)gridDim.y * kStoreCells) {
+    double w[kStoreCells];
+#pragma unroll
+    for (int q = 0; q < kStoreCells; q++) w[q] = cell + q < ncells ? W[(cell + q) * ncw + c] : 0.0;
+#pragma unroll
+    for (int q = 0; q < kStoreCells; q++)
+      if (cell + q < ncells) store_coef<ST>(table, (cell + q) * zs + tcol, w[q], iv);
+  }
 }
 
 __global__ void k_fill_f32(float *p, int64_t n, float v) {
@@ -499,7 +510,11 @@ Table *table_create(char kind, const GridDesc g[3], int num_splines, int storage
     pack_line_factors(f, one);
     t->factor_off[a] = all.size();
     all.insert(all.end(), one.begin(), one.end());
+    pack_fast_factors(f, one);
+    t->fast_off[a] = all.size();
+    all.insert(all.end(), one.begin(), one.end());
   }
+  t->fast_solve = fast_solve_fits(t);
   if (cudaMalloc(&t->factors_d, all.size() * sizeof(double)) != cudaSuccess ||
       cudaMemcpy(t->factors_d, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
     cudaGetLastError();
@@ -510,7 +525,7 @@ Table *table_create(char kind, const GridDesc g[3], int num_splines, int storage
   // Splines per batched solve: FP64 work space bounded by a budget.
   const double pts = (double)t->M[0] * t->M[1] * t->M[2];
   const double cells = (double)t->Nc[0] * t->Nc[1] * t->Nc[2];
-  const double per = t->ncomp * (pts * t->in_bytes + pts * 8.0 + cells * 8.0);
+  const double per = t->ncomp * (pts * t->in_bytes + (t->fast_solve ? 0.0 : pts * 8.0) + cells * 8.0);
   double budget = 4.0 * 1024 * 1024 * 1024;
   if (const char *env = getenv("EINSPLINE_GB300_SOLVE_BUDGET_MB")) budget = atof(env) * 1024.0 * 1024.0;
   t->cap = (int)std::max(1.0, std::min((double)num_splines, floor(budget / per)));
@@ -556,7 +571,7 @@ static int ensure_work(Table *t) {
   const size_t cells = (size_t)t->Nc[0] * t->Nc[1] * t->Nc[2];
   const size_t ncw = (size_t)t->cap * t->ncomp;
   cudaError_t e1 = cudaMalloc(&t->staging, pts * ncw * t->in_bytes);
-  cudaError_t e2 = cudaMalloc(&t->work_a, pts * ncw * sizeof(double));
+  cudaError_t e2 = cudaMalloc(&t->work_a, (t->fast_solve ? 1 : pts) * ncw * sizeof(double));
   cudaError_t e3 = cudaMalloc(&t->work_w, cells * ncw * sizeof(double));
   cudaError_t e4 = cudaMalloc(&t->colmax, ncw * sizeof(double));
   cudaError_t e5 = cudaMalloc(&t->slot_spline_d, t->cap * sizeof(int));
@@ -584,74 +599,88 @@ static int flush_locked(Table *t, const AxisOverride *ov = nullptr) {
   const int Nx = t->Nc[0], Ny = t->Nc[1], Nz = t->Nc[2];
   cudaStream_t s = t->stream;
   EG_CUDA(cudaMemcpyAsync(t->slot_spline_d, t->pend_spline.data(), n * sizeof(int), cudaMemcpyHostToDevice, s));
-  // 1. transpose queued data to spline-fastest FP64
-  dim3 tb(32, 8), tg((unsigned)((P + 31) / 32), (unsigned)((n + 31) / 32));
-  if (t->in_bytes == 4) {
-    if (nc == 1) k_stage_transpose<float, 1><<<tg, tb, 0, s>>>((const float *)t->staging, P, n, t->work_a);
-    else k_stage_transpose<float, 2><<<tg, tb, 0, s>>>((const float *)t->staging, P, n, t->work_a);
-  } else {
-    if (nc == 1) k_stage_transpose<double, 1><<<tg, tb, 0, s>>>((const double *)t->staging, P, n, t->work_a);
-    else k_stage_transpose<double, 2><<<tg, tb, 0, s>>>((const double *)t->staging, P, n, t->work_a);
-  }
-  count_launch();
-  EG_CUDA(cudaGetLastError());
-  // 2. sweeps: x (A -> W), then y and z in place on W
-  const int64_t wz = ncw, wy = (int64_t)Nz * ncw, wx = (int64_t)Ny * Nz * ncw;
-  const int64_t az = ncw, ay = (int64_t)Mz * ncw, ax = (int64_t)My * Mz * ncw;
   const int TB = 128;
   const int cblocks = (ncw + TB - 1) / TB;
-  for (int axis = 0; axis < t->dims; axis++) {
-    SweepArgs a;
-    memset(&a, 0, sizeof(a));
-    a.fac = t->factors_d + t->factor_off[axis];
-    a.ncw = ncw;
-    a.ncomp = nc;
-    for (int p = 0; p < 2; p++) { a.lval[p] = t->lval[axis][p]; a.rval[p] = t->rval[axis][p]; }
-    if (ov && axis == 0) {
-      a.fac = ov->fac;
-      for (int p = 0; p < 2; p++) { a.lval[p] = ov->lval[p]; a.rval[p] = ov->rval[p]; }
-    }
-    if (axis == 0) {
-      a.in = t->work_a; a.out = t->work_w;
-      a.nv = Mz; a.nlines = (int64_t)My * Mz;
-      a.in_su = ay; a.in_sv = az; a.out_su = wy; a.out_sv = wz;
-      a.in_stride = ax; a.out_stride = wx;
-    } else if (axis == 1) {
-      a.in = t->work_w; a.out = t->work_w;
-      a.nv = Mz; a.nlines = (int64_t)Nx * Mz;
-      a.in_su = wx; a.in_sv = wz; a.out_su = wx; a.out_sv = wz;
-      a.in_stride = wy; a.out_stride = wy;
+  if (t->fast_solve) {
+    if (int r = solve_fast(t, n, s)) return r;
+  } else {
+    // 1. transpose queued data to spline-fastest FP64
+    dim3 tb(32, 8), tg((unsigned)((P + 31) / 32), (unsigned)((n + 31) / 32));
+    if (t->in_bytes == 4) {
+      if (nc == 1) k_stage_transpose<float, 1><<<tg, tb, 0, s>>>((const float *)t->staging, P, n, t->work_a);
+      else k_stage_transpose<float, 2><<<tg, tb, 0, s>>>((const float *)t->staging, P, n, t->work_a);
     } else {
-      a.in = t->work_w; a.out = t->work_w;
-      a.nv = Ny; a.nlines = (int64_t)Nx * Ny;
-      a.in_su = wx; a.in_sv = wy; a.out_su = wx; a.out_sv = wy;
-      a.in_stride = wz; a.out_stride = wz;
+      if (nc == 1) k_stage_transpose<double, 1><<<tg, tb, 0, s>>>((const double *)t->staging, P, n, t->work_a);
+      else k_stage_transpose<double, 2><<<tg, tb, 0, s>>>((const double *)t->staging, P, n, t->work_a);
     }
-    const int64_t blocks = a.nlines * cblocks;
-    k_sweep<<<(unsigned)blocks, TB, 0, s>>>(a);
     count_launch();
     EG_CUDA(cudaGetLastError());
+    // 2. sweeps: x (A -> W), then y and z in place on W
+    const int64_t wz = ncw, wy = (int64_t)Nz * ncw, wx = (int64_t)Ny * Nz * ncw;
+    const int64_t az = ncw, ay = (int64_t)Mz * ncw, ax = (int64_t)My * Mz * ncw;
+    for (int axis = 0; axis < t->dims; axis++) {
+      SweepArgs a;
+      memset(&a, 0, sizeof(a));
+      a.fac = t->factors_d + t->factor_off[axis];
+      a.ncw = ncw;
+      a.ncomp = nc;
+      for (int p = 0; p < 2; p++) { a.lval[p] = t->lval[axis][p]; a.rval[p] = t->rval[axis][p]; }
+      if (ov && axis == 0) {
+        a.fac = ov->fac;
+        for (int p = 0; p < 2; p++) { a.lval[p] = ov->lval[p]; a.rval[p] = ov->rval[p]; }
+      }
+      if (axis == 0) {
+        a.in = t->work_a; a.out = t->work_w;
+        a.nv = Mz; a.nlines = (int64_t)My * Mz;
+        a.in_su = ay; a.in_sv = az; a.out_su = wy; a.out_sv = wz;
+        a.in_stride = ax; a.out_stride = wx;
+      } else if (axis == 1) {
+        a.in = t->work_w; a.out = t->work_w;
+        a.nv = Mz; a.nlines = (int64_t)Nx * Mz;
+        a.in_su = wx; a.in_sv = wz; a.out_su = wx; a.out_sv = wz;
+        a.in_stride = wy; a.out_stride = wy;
+      } else {
+        a.in = t->work_w; a.out = t->work_w;
+        a.nv = Ny; a.nlines = (int64_t)Nx * Ny;
+        a.in_su = wx; a.in_sv = wy; a.out_su = wx; a.out_sv = wy;
+        a.in_stride = wz; a.out_stride = wz;
+      }
+      const int64_t blocks = a.nlines * cblocks;
+      k_sweep<<<(unsigned)blocks, TB, 0, s>>>(a);
+      count_launch();
+      EG_CUDA(cudaGetLastError());
+    }
   }
   // 3. scales for 16-bit storage, 4. rounded store into the table columns
   const int64_t ncells = (int64_t)Nx * Ny * Nz;
   double *inv = reinterpret_cast<double *>(t->work_a);  // work_a is free again
   if (is16(t->storage)) {
-    EG_CUDA(cudaMemsetAsync(t->colmax, 0, ncw * sizeof(unsigned int), s));
-    dim3 cg((ncw + TB - 1) / TB, (unsigned)std::min<int64_t>(ncells, 1024));
-    k_colmax<<<cg, TB, 0, s>>>(t->work_w, ncells, ncw, (unsigned int *)t->colmax);
+    if (!t->fast_solve) {  // solve_fast finds the largest magnitudes on its way
+      EG_CUDA(cudaMemsetAsync(t->colmax, 0, ncw * sizeof(unsigned int), s));
+      dim3 cg((ncw + TB - 1) / TB, (unsigned)std::min<int64_t>(ncells, 1024));
+      k_colmax<<<cg, TB, 0, s>>>(t->work_w, ncells, ncw, (unsigned int *)t->colmax);
+      count_launch();
+    }
     k_scales<<<(n + 127) / 128, 128, 0, s>>>(t->storage, (const unsigned int *)t->colmax, n, nc, t->slot_spline_d,
                                              t->scale, inv);
-    count_launch(2);
+    count_launch();
     EG_CUDA(cudaGetLastError());
   }
-  const int64_t sblocks = ncells * cblocks;
-  switch (t->storage) {
-    case ST_F64: k_store<ST_F64><<<(unsigned)sblocks, TB, 0, s>>>(t->work_w, ncells, ncw, nc, t->slot_spline_d, inv, t->coefs, t->zs); break;
-    case ST_F32: k_store<ST_F32><<<(unsigned)sblocks, TB, 0, s>>>(t->work_w, ncells, ncw, nc, t->slot_spline_d, inv, t->coefs, t->zs); break;
-    case ST_F16: k_store<ST_F16><<<(unsigned)sblocks, TB, 0, s>>>(t->work_w, ncells, ncw, nc, t->slot_spline_d, inv, t->coefs, t->zs); break;
-    case ST_I16: k_store<ST_I16><<<(unsigned)sblocks, TB, 0, s>>>(t->work_w, ncells, ncw, nc, t->slot_spline_d, inv, t->coefs, t->zs); break;
-    default: k_store<ST_BF16><<<(unsigned)sblocks, TB, 0, s>>>(t->work_w, ncells, ncw, nc, t->slot_spline_d, inv, t->coefs, t->zs); break;
+  if (t->fast_solve && t->storage == ST_F32) {  // the z solve wrote the table
+    t->pend_spline.clear();
+    t->slot_of.clear();
+    return 0;
   }
+  const dim3 sg((unsigned)cblocks, (unsigned)std::min<int64_t>((ncells + kStoreCells - 1) / kStoreCells, 16384));
+#define EG_STORE(ST) k_store<ST><<<sg, TB, 0, s>>>(t->work_w, ncells, ncw, nc, t->slot_spline_d, inv, t->coefs, t->zs)
+  switch (t->storage) {
+    case ST_F64: EG_STORE(ST_F64); break;
+    case ST_F32: EG_STORE(ST_F32); break;
+    case ST_F16: EG_STORE(ST_F16); break;
+    case ST_I16: EG_STORE(ST_I16); break;
+    default: EG_STORE(ST_BF16); break;
+  }
+#undef EG_STORE
   count_launch();
   EG_CUDA(cudaGetLastError());
   t->pend_spline.clear();
@@ -767,6 +796,17 @@ int table_set(Table *t, int first, int count, const void *data, bool from_device
   std::lock_guard<std::mutex> g(t->mu);
   if (int r = ensure_work(t)) return r;
   const size_t per = (size_t)t->M[0] * t->M[1] * t->M[2] * t->ncomp * t->in_bytes;
+  // Neighbouring splines in neighbouring slots go in one copy (a separate
+  // copy per spline kept the host busy for 4 us each: 2 ms of the 12 ms that
+  // set + flush of 64^3 x 512 took).
+  int run_slot = 0, run_first = 0, run_n = 0;
+  auto copy_run = [&]() -> int {
+    if (run_n)
+      EG_CUDA(cudaMemcpyAsync((char *)t->staging + (size_t)run_slot * per, (const char *)data + (size_t)run_first * per,
+                              per * run_n, from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, t->stream));
+    run_n = 0;
+    return 0;
+  };
   for (int i = 0; i < count; i++) {
     const int sp = first + i;
     int slot;
@@ -774,17 +814,23 @@ int table_set(Table *t, int first, int count, const void *data, bool from_device
     if (it != t->slot_of.end()) {
       slot = it->second;
     } else {
-      if ((int)t->pend_spline.size() == t->cap)
+      if ((int)t->pend_spline.size() == t->cap) {
+        if (int r = copy_run()) return r;
         if (int r = flush_locked(t)) return r;
+      }
       slot = (int)t->pend_spline.size();
       t->pend_spline.push_back(sp);
       t->slot_of[sp] = slot;
     }
-    const char *src = (const char *)data + (size_t)i * per;
-    EG_CUDA(cudaMemcpyAsync((char *)t->staging + (size_t)slot * per, src, per,
-                            from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, t->stream));
+    if (run_n && slot != run_slot + run_n)
+      if (int r = copy_run()) return r;
+    if (!run_n) {
+      run_slot = slot;
+      run_first = i;
+    }
+    run_n++;
   }
-  return 0;
+  return copy_run();
 }
 
 // ------------------------------------------------------------------
