@@ -17,13 +17,19 @@
 // are deterministic.  k_det_tc does the same for F16 and BF16 tables on the
 // tensor cores (their default load mode 5).
 //
-// The update is two passes over each accepted walker's inverse:
+// The update (k_det_update; matrices above kUpMax by separate kernels, one
+// a pass) is two passes over each accepted walker's inverse:
 //   pass 1: x = delta^T Ainv (delta = u - A[k,:]) and colk = Ainv[:,k];
 //   pass 2: Ainv += (-1 / (1 + x[k])) colk x^T, A[k,:] = u.
 // Unlike the reference's kernel 1, where every block of a walker writes the
 // new row into A while other blocks still read the old one, A is only read in
 // pass 1 and written in pass 2.
 #include <string.h>
+
+#include <algorithm>
+#include <map>
+#include <mutex>
+#include <tuple>
 
 #include "eval_core.h"
 
@@ -553,6 +559,336 @@ __global__ void __launch_bounds__(kTcThreads, kDtBlocksPerSM) k_det_tc(const __g
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(RA * NC) : "memory");
 }
 
+// ------------------------------------------------------------ fused update
+// Accepted walkers' updates, each by one thread-block cluster: the CTAs
+// split the stored rows of the inverse, read them for x and column k, exchange
+// over distributed shared memory, and read them again for the rank-1
+// correction while they are still in L2.  The two passes below move 3 N^2
+// floats a walker through DRAM, this 2 N^2.  Clusters stay and take walker
+// after walker.
+//
+// The rows stream through a ring of kUpDepth 16-byte asynchronous copies a
+// thread, in order: a walker's rows, the same rows again, the next walker's.
+// A thread reads back only what it copied itself, so the stream needs no
+// barrier, and the copies in flight (64 KB for 512 threads) keep DRAM busy
+// while the cluster exchanges.  Bound by DRAM: 768 x 768, 512 walkers: 488 us
+// (two passes 1098 us), 2.78 GB at 5.8 TB/s, of which 0.4 GB are rows that
+// had left L2; launch shapes and figures at update_shape.
+//
+// Reference layout (TRANS 0, rows are orbitals): every CTA sums its rows'
+// share of x for all columns, and every CTA adds all shares in rank order.
+// A thread owns a unit of 4 columns and every G-th row of its CTA.
+// Transposed layout (rows are electrons): x[c] is the dot product of row c
+// with delta, found and used by the same CTA; column k is stored row k, which
+// every CTA reads before its owner changes it.  2^lpr_log lanes share a row.
+//
+// Sums run in a fixed order: results do not vary from run to run.
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+// The float at shared-memory address a (of this CTA) in CTA `rank` of the cluster.
+__device__ __forceinline__ float ld_cluster(unsigned a, unsigned rank) {
+  float v;
+  asm volatile(
+      "{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}"
+      : "=f"(v)
+      : "r"(a), "r"(rank)
+      : "memory");
+  return v;
+}
+
+constexpr int kUpVec = 4;    // entries of a walker's vectors a thread: n <= kUpVec * THREADS
+constexpr int kUpDepth = 8;  // items in flight a thread
+
+// Shared memory: the ring, then floats -- the new row's own entries; TRANS 0:
+// the own rows' delta and column k, this CTA's share of x, x, partial sums of
+// the row groups; TRANS 1: delta, column k, the own rows' x.
+__host__ __device__ __forceinline__ int up4(int n) { return (n + 3) & ~3; }
+__host__ __device__ __forceinline__ size_t up_smem(int n, int cs, int trans, int threads) {
+  const size_t n4 = up4(n), own = up4((n + cs - 1) / cs);
+  const size_t part = n4 > (size_t)(4 * threads) ? n4 : 4 * threads;
+  return (size_t)kUpDepth * threads * 16 + 4 * (trans ? 2 * n4 + 2 * own : 3 * own + 2 * n4 + part);
+}
+
+template <int TRANS, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_det_update(const DetArgs d, int cs, int naccept, int lpr_log) {
+  extern __shared__ __align__(16) unsigned char up_raw[];
+  constexpr int D = kUpDepth;
+  constexpr unsigned kSlot = THREADS * 16;
+  float *up = reinterpret_cast<float *>(up_raw + D * kSlot);
+  const int n = d.n, tid = threadIdx.x;
+  const int U = (n + 3) >> 2, n4 = up4(n), own = (n + cs - 1) / cs, ownp = up4(own);
+  const unsigned rank = cluster_rank();
+  const int step = gridDim.x / cs;
+  const int r0 = (int)((int64_t)n * rank / cs), r1 = (int)((int64_t)n * (rank + 1) / cs);
+  // A pass over the own rows takes QN x R items a thread, the same for every
+  // thread, in whole rounds of D; this one has NQ x NR of them (TRANS 0: R
+  // rows of one unit; TRANS 1: QN rows of R units).
+  const int LPR = 1 << lpr_log;
+  const int G = TRANS ? THREADS >> lpr_log : THREADS / U;
+  const int g = TRANS ? tid >> lpr_log : tid / U;
+  const int q0 = TRANS ? tid & (LPR - 1) : tid % U;
+  const int QN = TRANS ? (own + G - 1) / G : 1;
+  const int R = TRANS ? (U + LPR - 1) >> lpr_log : (own + G - 1) / G;
+  const int rounds = (QN * R + D - 1) / D;
+  const int rows = g < G && r0 + g < r1 ? (r1 - r0 - g + G - 1) / G : 0;
+  const int NQ = TRANS ? rows : 1, NR = TRANS ? (U - q0 + LPR - 1) >> lpr_log : rows;
+  const int64_t first = (int64_t)(r0 + g) * d.ld + 4 * q0;      // the first item's place in the matrix
+  const int64_t inner = TRANS ? 4 * LPR : (int64_t)G * d.ld;    // from item to item
+  const int64_t outer = TRANS ? (int64_t)G * d.ld - (int64_t)R * inner : 0;  // further after R items (TRANS 1)
+  const int tail = n & 3;                                       // columns of the last unit, when not 4
+  const bool rows16 = (d.ld & 3) == 0;                          // every row as aligned as the first
+
+  // the stream's issue side: the next round's walker, pass and items
+  const float *ibase = nullptr, *inext = nullptr, *isrc = nullptr;
+  int iw = blockIdx.x / cs, iround = 0, iq = 0, ir = 0, ipass = 0;
+  bool ivec = false;
+  auto enter_walker = [&](const float *base) {
+    ibase = base;
+    ivec = rows16 && al16(base);
+    isrc = base + first;
+    if (iw + step < naccept) inext = d.ainv[iw + step];
+  };
+  if (iw < naccept) enter_walker(d.ainv[iw]);
+  else ir = NR;  // nothing to copy
+  const unsigned ring = (unsigned)__cvta_generic_to_shared(up_raw) + tid * 16;
+  auto issue = [&](int q) {  // one item into slot q
+    if (TRANS ? ir < NR && iq < NQ : ir < NR) {
+      const unsigned dst = ring + q * kSlot;
+      if (ivec) {  // a last unit of fewer columns reads on into its row's padding
+        cp_async<16>(dst, reinterpret_cast<const char *>(isrc));
+      } else {
+        const int e1 = tail && q0 + (TRANS ? ir << lpr_log : 0) == U - 1 ? tail : 4;
+        for (int e = 0; e < e1; e++) cp_async<4>(dst + 4 * e, reinterpret_cast<const char *>(isrc + e));
+      }
+    }
+    cp_async_commit();
+    isrc += inner;
+    ir++;
+    if (TRANS && ir == R) {
+      ir = 0;
+      iq++;
+      isrc += outer;
+    }
+  };
+  auto next_round = [&]() {
+    if (++iround < rounds) return;
+    iround = iq = ir = 0;
+    if ((ipass ^= 1) == 0) {
+      iw += step;
+      if (iw < naccept) enter_walker(inext);
+    }
+    if (iw < naccept) isrc = ibase + first;
+    else { ir = NR; iq = NQ; }
+  };
+#pragma unroll
+  for (int q = 0; q < D; q++) issue(q);
+  next_round();
+  // the item in slot q, the oldest in flight
+  auto take = [&](int q) {
+    cp_async_wait<D - 1>();
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(ring + q * kSlot)
+                 : "memory");
+    return v;
+  };
+
+  float *unew = up, *delta = up + ownp, *ck = delta + (TRANS ? n4 : ownp), *sx = ck + (TRANS ? n4 : ownp);
+  float *xf = sx + n4, *part = xf + n4;  // TRANS 0
+  // The vectors a walker needs beside its rows (u and A's row k -- the own
+  // entries, or for TRANS all of them and stored row k) are read into
+  // registers a walker ahead, so that no wait for them is exposed.
+  const int v0 = TRANS ? 0 : r0, v1 = TRANS ? n : r1;
+  float vu[kUpVec], va[kUpVec], vk[TRANS ? kUpVec : 1];
+  int w = blockIdx.x / cs;
+  const float *pu = nullptr, *pa = nullptr, *pm = nullptr;
+  auto addresses = [&](int wk) {
+    if (wk < naccept) { pu = d.urow[wk]; pa = d.amat[wk]; pm = d.ainv[wk]; }
+  };
+  auto read_vectors = [&]() {
+#pragma unroll
+    for (int i = 0; i < kUpVec; i++) {
+      const int j = v0 + tid + i * THREADS;
+      if (j < v1) {
+        vu[i] = pu[j];
+        va[i] = pa[(int64_t)d.k * d.ld + j];
+        if (TRANS) vk[TRANS ? i : 0] = pm[(int64_t)d.k * d.ld + j];
+      }
+    }
+  };
+  addresses(w);
+  if (w < naccept) read_vectors();
+  const unsigned sxa = (unsigned)__cvta_generic_to_shared(sx);
+  const int kc = !TRANS && q0 == d.k >> 2 ? d.k & 3 : -1;  // the component of this thread's unit in column k
+  for (; w < naccept; w += step) {
+    float *m = const_cast<float *>(pm), *arow = const_cast<float *>(pa) + (int64_t)d.k * d.ld;
+    const bool vec = rows16 && al16(m);
+    __syncthreads();  // the last walker's vectors are no longer read
+#pragma unroll
+    for (int i = 0; i < kUpVec; i++) {
+      const int j = v0 + tid + i * THREADS;
+      if (j < v1) {
+        delta[j - v0] = vu[i] - va[i];
+        if (TRANS) ck[j] = vk[TRANS ? i : 0];
+        if (!TRANS || (j >= r0 && j < r1)) unew[j - r0] = vu[i];
+      } else if (TRANS && j < n4) {
+        delta[j] = ck[j] = 0.f;
+      }
+    }
+    addresses(w + step);
+    __syncthreads();
+    // pass 1: x
+    if constexpr (TRANS) {
+      int qi = 0, ri = 0;
+      float s = 0.f;
+      for (int c = 0; c < rounds; c++) {
+#pragma unroll
+        for (int q = 0; q < D; q++) {
+          float4 v = take(q);
+          if (ri < NR && qi < NQ) {
+            const int unit = q0 + (ri << lpr_log);
+            if (tail && unit == U - 1) {  // what lies past the row's end does not count, not even as 0 * NaN
+              v.w = 0.f;
+              if (tail < 3) v.z = 0.f;
+              if (tail < 2) v.y = 0.f;
+            }
+            const float4 de = *reinterpret_cast<const float4 *>(delta + 4 * unit);
+            s = fmaf(v.x, de.x, s); s = fmaf(v.y, de.y, s);
+            s = fmaf(v.z, de.z, s); s = fmaf(v.w, de.w, s);
+          }
+          issue(q);
+          if (++ri == R) {
+            for (int off = LPR >> 1; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+            if (q0 == 0 && qi < NQ) sx[g + qi * G] = s;
+            s = 0.f;
+            ri = 0;
+            qi++;
+          }
+        }
+        next_round();
+      }
+    } else {
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      const float *de = delta + g;
+      float *cp = ck + g;
+      int left = NR;
+      for (int c = 0; c < rounds; c++, left -= D) {
+#pragma unroll
+        for (int q = 0; q < D; q++, de += G, cp += G) {
+          const float4 v = take(q);
+          if (q < left) {
+            const float x = *de;
+            if (kc >= 0) *cp = kc == 0 ? v.x : kc == 1 ? v.y : kc == 2 ? v.z : v.w;
+            acc.x = fmaf(v.x, x, acc.x); acc.y = fmaf(v.y, x, acc.y);
+            acc.z = fmaf(v.z, x, acc.z); acc.w = fmaf(v.w, x, acc.w);
+          }
+          issue(q);
+        }
+        next_round();
+      }
+      if (g < G) *reinterpret_cast<float4 *>(part + g * n4 + 4 * q0) = acc;
+    }
+    __syncthreads();
+    if (!TRANS) {
+      for (int c = tid; c < n; c += THREADS) {
+        float s = part[c];
+        for (int i = 1; i < G; i++) s += part[i * n4 + c];
+        sx[c] = s;
+      }
+    }
+    // the shares of x are ready; A's row k and stored row k have been read
+    cluster_arrive();
+    cluster_wait();
+    if (TRANS) {
+      const int kown = (int)((((int64_t)d.k + 1) * cs - 1) / n);  // the CTA that holds row k
+      const float p = -1.0f / (1.0f + ld_cluster(sxa + 4 * (d.k - (int)((int64_t)n * kown / cs)), kown));
+      for (int j = tid; j < n; j += THREADS) ck[j] *= p;
+    } else {
+      for (int c = tid; c < n4; c += THREADS) {
+        float s = 0.f;
+        if (c < n) {
+          float t[8];  // clusters of at most 8: all reads in flight at once
+#pragma unroll
+          for (int i = 0; i < 8; i++) t[i] = i < cs ? ld_cluster(sxa + 4 * c, i) : 0.f;
+#pragma unroll
+          for (int i = 0; i < 8; i++) s += t[i];
+        }
+        xf[c] = s;
+      }
+    }
+    cluster_arrive();  // this CTA is done with the others' shared memory
+    for (int j = r0 + tid; j < r1; j += THREADS) arow[j] = unew[j - r0];
+    __syncthreads();
+    if (w + step < naccept) read_vectors();
+    // pass 2: the correction
+    float *dst = m + first;
+    auto put = [&](float4 v, int unit) {
+      const bool whole = tail == 0 || unit != U - 1;
+      if (vec && whole) {
+        __stcs(reinterpret_cast<float4 *>(dst), v);
+      } else {
+        dst[0] = v.x;
+        if (whole || tail > 1) dst[1] = v.y;
+        if (whole || tail > 2) dst[2] = v.z;
+        if (whole) dst[3] = v.w;
+      }
+    };
+    if constexpr (TRANS) {
+      int qi = 0, ri = 0;
+      float xr = NQ > 0 ? sx[g] : 0.f;
+      for (int c = 0; c < rounds; c++) {
+#pragma unroll
+        for (int q = 0; q < D; q++) {
+          float4 v = take(q);
+          if (ri < NR && qi < NQ) {
+            const int unit = q0 + (ri << lpr_log);
+            const float4 c4 = *reinterpret_cast<const float4 *>(ck + 4 * unit);
+            v.x = fmaf(xr, c4.x, v.x); v.y = fmaf(xr, c4.y, v.y);
+            v.z = fmaf(xr, c4.z, v.z); v.w = fmaf(xr, c4.w, v.w);
+            put(v, unit);
+          }
+          issue(q);
+          dst += inner;
+          if (++ri == R) {
+            ri = 0;
+            qi++;
+            dst += outer;
+            if (qi < NQ) xr = sx[g + qi * G];
+          }
+        }
+        next_round();
+      }
+    } else {
+      const float p = -1.0f / (1.0f + xf[d.k]);
+      const float4 x = *reinterpret_cast<const float4 *>(xf + 4 * q0);
+      const float *cp = ck + g;
+      int left = NR;
+      for (int c = 0; c < rounds; c++, left -= D) {
+#pragma unroll
+        for (int q = 0; q < D; q++, cp += G, dst += inner) {
+          float4 v = take(q);
+          if (q < left) {
+            const float rs = p * *cp;
+            v.x = fmaf(x.x, rs, v.x); v.y = fmaf(x.y, rs, v.y);
+            v.z = fmaf(x.z, rs, v.z); v.w = fmaf(x.w, rs, v.w);
+            put(v, q0);
+          }
+          issue(q);
+        }
+        next_round();
+      }
+    }
+    cluster_wait();
+  }
+  cp_async_wait<0>();
+}
+
 // Pass 1, reference layout (Ainv[j][c] row-major): thread per column c,
 // rows streamed in order with delta staged in shared memory; the thread that
 // owns column k also copies that column out.
@@ -673,6 +1009,89 @@ int num_sms() {
     return 152;
   }
   return n;
+}
+
+// The fused update's launch, by the matrix size.  Larger clusters keep fewer
+// matrices in flight, so that a walker's rows are still in L2 when they are
+// read again (measured: all of them up to 45 MB in flight, two thirds at
+// 85 MB); smaller blocks and clusters spend less on each walker's
+// exchange, which is what bounds small matrices.  us an update of about 1 GB
+// of inverses (16000 walkers for n = 64, 0.26 GB), reference / transposed
+// layout, the line's own shape in brackets, and the two passes:
+//          1 x 128    2 x 128    2 x 256    8 x 128    8 x 256    8 x 512   passes
+//   n 64  [125/144]   166/222    281/402                                   484/453
+//    160   396/402   [318/412]   322/--                                    850/768
+//    200    --/499    430/435   [357/480]   456/530                        965/850
+//    256                         --         [378/400]              696/1035 877/710
+//    384              561/560    508/570     446/456   [400/452]   528/669  913/643
+//    512                         --          533/533    417/455   [413/448] 843/616
+//    768                                                           [498/506] 1097/665
+//   2048                                                           [517/515] 1260/557
+// Beyond kUpMax a matrix no longer fits the vectors' registers.
+struct UpdateShape {
+  int cs, threads;
+};
+constexpr int kUpMax = 2048;
+UpdateShape update_shape(int n) {
+  if (n <= 100) return {1, 128};
+  if (n <= 160) return {2, 128};
+  if (n <= 240) return {2, 256};
+  if (n <= 360) return {8, 128};
+  if (n <= 500) return {8, 256};
+  return {8, 512};
+}
+
+template <int THREADS>
+const void *update_kernel(int trans) {
+  return trans ? (const void *)k_det_update<1, THREADS> : (const void *)k_det_update<0, THREADS>;
+}
+
+cudaLaunchConfig_t cluster_config(int blocks, int cs, int threads, size_t smem, cudaStream_t s,
+                                  cudaLaunchAttribute *at) {
+  cudaLaunchConfig_t lc;
+  memset(&lc, 0, sizeof(lc));
+  lc.gridDim = dim3((unsigned)blocks);
+  lc.blockDim = dim3((unsigned)threads);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = s;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = (unsigned)cs;
+  at->val.clusterDim.y = at->val.clusterDim.z = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return lc;
+}
+
+// Clusters of a kernel that the current device holds at once (0: none, or
+// the query failed), looked up once per kernel, shape and device; the
+// kernel's shared-memory limit is raised to most, its largest launch's.
+int resident_clusters(const void *func, int cs, int threads, size_t smem, size_t most) {
+  struct Key {
+    const void *f;
+    int cs, threads, dev;
+    size_t smem;
+    bool operator<(const Key &o) const {
+      return std::tie(f, cs, threads, dev, smem) < std::tie(o.f, o.cs, o.threads, o.dev, o.smem);
+    }
+  };
+  static std::mutex mu;
+  static std::map<Key, int> cache;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return 0; }
+  const Key k{func, cs, threads, dev, smem};
+  std::lock_guard<std::mutex> g(mu);
+  auto it = cache.find(k);
+  if (it != cache.end()) return it->second;
+  int fit = 0;
+  cudaLaunchAttribute at;
+  const cudaLaunchConfig_t lc = cluster_config(cs, cs, threads, smem, nullptr, &at);
+  if ((most > 48 * 1024 &&
+       cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) ||
+      cudaOccupancyMaxActiveClusters(&fit, func, &lc) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return cache[k] = fit;
 }
 
 int check_det_opts(const einspline_gb300_det_opts *o, const char *fn) {
@@ -813,6 +1232,26 @@ int einspline_gb300_det_update(const einspline_gb300_det_opts *o, int naccept, f
   d.ld = o->ld;
   d.trans = o->ainv_trans;
   cudaStream_t s = stream ? (cudaStream_t)stream : cudaStreamLegacy;
+  if (d.n <= kUpMax) {
+    const UpdateShape sh = update_shape(d.n);
+    const void *f = sh.threads == 128 ? update_kernel<128>(d.trans)
+                  : sh.threads == 256 ? update_kernel<256>(d.trans) : update_kernel<512>(d.trans);
+    const size_t sm = up_smem(d.n, sh.cs, d.trans, sh.threads);
+    const size_t most = up_smem(std::min(kUpMax, kUpVec * sh.threads), sh.cs, d.trans, sh.threads);
+    const int fit = resident_clusters(f, sh.cs, sh.threads, sm, most);
+    if (fit > 0) {
+      const int clusters = std::min(naccept, fit);
+      int lpr_log = 0;
+      while (lpr_log < 5 && (1 << lpr_log) < (d.n + 3) / 4) lpr_log++;
+      int cs = sh.cs;
+      void *args[] = {&d, &cs, &naccept, &lpr_log};
+      cudaLaunchAttribute at;
+      const cudaLaunchConfig_t lc = cluster_config(clusters * cs, cs, sh.threads, sm, s, &at);
+      EG_CUDA(cudaLaunchKernelExC(&lc, f, args));
+      count_launch();
+      return 0;
+    }
+  }
   if (!d.trans) k_det_update1_rows<<<dim3((d.n + 255) / 256, naccept), 256, 0, s>>>(d);
   else k_det_update1_trans<<<dim3((d.n + 7) / 8, naccept), 256, 0, s>>>(d);
   EG_CUDA(cudaGetLastError());
