@@ -256,6 +256,129 @@ int sort_points(Table *t, const EvalArgs &a, int **perm_out, cudaStream_t s) {
   return 0;
 }
 
+// ------------------------------------------------------- points in open order
+// Random-order launches of a large batch on a large table read each stencil
+// row from DRAM once per point that uses it; in cell order, once.  So such a
+// launch sorts first, as opts.sort does, with the same bits as a result.
+//
+// When it pays: a sort costs 10-12 us.  With n points on R rows, random
+// order reads 64 n rows and cell order about R (1 - exp(-64 n / R)).  Measured
+// on GB300, vgh unless noted, us a launch in random / cell order (sort
+// included), by table and bytes saved:
+//   1231 MB  64^3 x 1024 FP32   0.10 GB  93/100   0.34 GB 172/158   1.1 GB  333/257   3.0 GB  657/433
+//    615 MB  64^3 x 1024 F16    0.17 GB  97/98    0.55 GB 185/151   1.5 GB  360/251   3.6 GB  708/448
+//    615 MB  values, I16        0.17 GB  95/105   0.55 GB 144/121   1.5 GB  281/193
+//    615 MB  vgh, I16           0.55 GB 202/205   1.5 GB  387/379   3.6 GB  755/722
+//    271 MB  48^3 x 512 FP32    0.29 GB  78/86    0.78 GB 138/129   1.8 GB  265/227
+//    162 MB  40^3 x 1024 F16    0.37 GB  79/81    values 1.9 GB 167/169
+//    135 MB  48^3 x 512 F16     0.39 GB  76/81    values 0.9 GB  85/99
+// Tables near the 129 MB L2 are mostly served by it in any order.  I16 vgh
+// is bound by its arithmetic, and FP64 tables by theirs: IEEE arithmetic
+// never gains, double-float only on values (154/135 at 0.58 GB).
+constexpr size_t kOrderTableBytes = 192u << 20;
+constexpr double kOrderSavedBytes = 0.5e9, kOrderSavedBytesI16 = 2e9;
+
+static bool order_pays(const Table *t, const EvalArgs &a, bool vgh) {
+  if (!t->order_dev || (t->storage == ST_F64 && (vgh || t->fp64_mode != 1))) return false;
+  const double R = (double)t->Nc[0] * t->Nc[1] * t->Nc[2], n64 = 64.0 * (double)a.npts;
+  const double saved = (n64 - R * (1.0 - exp(-n64 / R))) * (double)t->zs * t->elem_bytes;
+  return saved > (vgh && t->storage == ST_I16 ? kOrderSavedBytesI16 : kOrderSavedBytes);
+}
+
+void order_scratch_init(Table *t) {
+  if (t->dims != 3 || t->table_bytes < kOrderTableBytes) return;
+  const size_t piece = align_up_sz(small_sort_bytes(kSmallSort), 256);
+  bool ok = cudaMalloc(&t->order_dev, Table::kOrderSlots * piece) == cudaSuccess;
+  if (!ok) t->order_dev = nullptr;
+  for (auto &sl : t->order_slot)
+    ok = ok && cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming) == cudaSuccess;
+  if (ok) return;
+  cudaGetLastError();  // without scratch, launches keep their order
+  order_scratch_free(t);
+}
+
+void order_scratch_free(Table *t) {
+  cudaFree(t->order_dev);
+  t->order_dev = nullptr;
+  for (auto &sl : t->order_slot)
+    if (sl.done) {
+      cudaEventDestroy(sl.done);
+      sl.done = nullptr;
+    }
+}
+
+// The piece of scratch for a launch on s, or -1: the one s used last, else an
+// unused one, else one whose last launch is over.  The caller holds
+// order_mu.  Event queries run in relaxed capture mode, so that they do not
+// disturb a capture in another thread.
+static int order_piece(Table *t, cudaStream_t s) {
+  for (int i = 0; i < Table::kOrderSlots; i++)
+    if (t->order_slot[i].used && t->order_slot[i].stream == s) return i;
+  for (int i = 0; i < Table::kOrderSlots; i++)
+    if (!t->order_slot[i].used) return i;
+  int found = -1;
+  cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
+  if (cudaThreadExchangeStreamCaptureMode(&m) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  for (int i = 0; i < Table::kOrderSlots && found < 0; i++)
+    if (cudaEventQuery(t->order_slot[i].done) == cudaSuccess) found = i;
+  cudaGetLastError();  // cudaErrorNotReady is not an error
+  cudaThreadExchangeStreamCaptureMode(&m);
+  return found;
+}
+
+int launch_eval_ordered(Table *t, EvalArgs &a, bool vgh, cudaStream_t s) {
+  int tx, ty, pb;
+  auto plain = [&]() {
+    pick_tile(t, vgh, a.npts, tx, ty, pb);
+    return launch_eval(t, a, vgh, s, tx, ty, pb);
+  };
+  if (!order_pays(t, a, vgh)) return plain();
+  // a captured launch is replayed at times unknown here, when the scratch
+  // may hold another launch's order
+  cudaStreamCaptureStatus cap;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return plain();
+  }
+  if (cap != cudaStreamCaptureStatusNone) return plain();
+  std::lock_guard<std::mutex> lock(t->order_mu);
+  const int i = order_piece(t, s);
+  if (i < 0) return plain();
+  Table::OrderSlot &sl = t->order_slot[i];
+  // (a stream's handle may come back as another stream's)
+  if (sl.used) EG_CUDA(cudaStreamWaitEvent(s, sl.done, 0));
+  sl.used = true;
+  sl.stream = s;
+  void *piece = (char *)t->order_dev + (size_t)i * align_up_sz(small_sort_bytes(kSmallSort), 256);
+  const EvalArgs whole = a;
+  const size_t pos_b = 3 * (whole.pos_f64 ? 8 : 4), rb = t->storage == ST_F64 ? 8 : 4;
+  int r = 0;
+  for (int64_t p0 = 0; p0 < whole.npts && !r; p0 += kSmallSort) {
+    a = whole;
+    a.npts = std::min<int64_t>(kSmallSort, whole.npts - p0);
+    a.pos = (const char *)whole.pos + p0 * pos_b;
+    if (a.sign) a.sign = (const char *)whole.sign + p0 * rb;
+    if (a.vals_pp) a.vals_pp += p0;
+    if (a.grads_pp) a.grads_pp += p0;
+    if (a.hess_pp) a.hess_pp += p0;
+    if (a.vals) a.vals = (char *)whole.vals + p0 * whole.vstride * (int64_t)rb;
+    if (a.grads) a.grads = (char *)whole.grads + p0 * whole.gstride * (int64_t)rb;
+    if (a.hess) a.hess = (char *)whole.hess + p0 * whole.hstride * (int64_t)rb;
+    int *perm = nullptr;
+    r = small_sort_into(a, piece, &perm, s);
+    if (r) break;
+    a.perm = perm;
+    pick_tile(t, vgh, a.npts, tx, ty, pb, true);
+    r = launch_eval(t, a, vgh, s, tx, ty, pb);
+  }
+  const cudaError_t e = cudaEventRecord(sl.done, s);
+  if (!r && e != cudaSuccess) r = cuda_check(e, "evaluation in cell order");
+  return r;
+}
+
 // ------------------------------------------------------------------ helpers
 __global__ void k_scale_box(double *pos, int64_t n, double lx, double ly, double lz) {
   const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -289,11 +412,10 @@ static int eval_device(Table *t, const einspline_gb300_eval_opts *o, int64_t npt
   a.npts = npts;
   a.pos = pos_d;
   a.vals = v; a.grads = g; a.hess = h;
-  if (o->sort && npts > 1) {
-    int *perm = nullptr;
-    if (int r = sort_points(t, a, &perm, s)) return r;
-    a.perm = perm;
-  }
+  if (!o->sort || npts <= 1) return launch_eval_ordered(t, a, o->vgh != 0, s);
+  int *perm = nullptr;
+  if (int r = sort_points(t, a, &perm, s)) return r;
+  a.perm = perm;
   int tx, ty, pb;
   pick_tile(t, o->vgh != 0, npts, tx, ty, pb, a.perm != nullptr);
   return launch_eval(t, a, o->vgh != 0, s, tx, ty, pb);

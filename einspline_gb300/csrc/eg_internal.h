@@ -141,6 +141,19 @@ struct einspline_gb300_table {
   void *sort_dev = nullptr;
   size_t sort_bytes = 0;
 
+  // scratch in which random-order launches are put into cell order
+  // (launch_eval_ordered), kOrderSlots pieces, each used by one stream at a
+  // time; only on tables that such launches gain on (order_scratch_init)
+  struct OrderSlot {
+    cudaStream_t stream = nullptr;  // the last launch's, once used
+    bool used = false;
+    cudaEvent_t done = nullptr;     // after the last launch that read the piece
+  };
+  static constexpr int kOrderSlots = 4;
+  std::mutex order_mu;              // held while a launch is queued
+  void *order_dev = nullptr;
+  OrderSlot order_slot[kOrderSlots];
+
   // launch shape and load mode (-1: not forced)
   int tile_tx = 0, tile_ty = 0, tile_pb = 0, tile_mode = -1;
   // set by a TMA-staged evaluation whose bounded barrier wait ran out
@@ -269,6 +282,14 @@ int pick_mode(Table *t, bool vgh, bool sorted = false);
 // Tensor map of a 16-bit table for the tensor-core kernels (load mode 5).
 int tc_table_map(const Table *t, EvalArgs &a);
 int elems_per_thread(const Table *t);
+
+// A batched evaluation whose caller left the order of the points open:
+// launches it, in cell order when that pays (see api_ext.cu).  Picks the
+// launch shape itself; a.perm is null.
+int launch_eval_ordered(Table *t, EvalArgs &a, bool vgh, cudaStream_t s);
+// Table creation and destruction.
+void order_scratch_init(Table *t);
+void order_scratch_free(Table *t);
 
 // sorting
 int sort_points(Table *t, const EvalArgs &a, int **perm_out, cudaStream_t s);

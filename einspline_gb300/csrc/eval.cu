@@ -1437,9 +1437,7 @@ void eval_cuda(CS *c, const void *pos_d, bool pos_f64, void *const *vals_d, void
   a.linv = linv;
   a.lrow = lrow;
   if (out == 1 && (!linv || !grads_d)) { fail(EINSPLINE_GB300_EINVAL, "%s: Linv and grad_lapl are required", fn); return; }
-  int tx, ty, pb;
-  pick_tile(t, vgh, num, tx, ty, pb);
-  if (launch_eval(t, a, vgh, cudaStreamLegacy, tx, ty, pb)) return;
+  if (launch_eval_ordered(t, a, vgh, cudaStreamLegacy)) return;
   cudaError_t e = cudaStreamSynchronize(cudaStreamLegacy);
   if (e != cudaSuccess) cuda_check(e, fn);
 }

@@ -515,6 +515,7 @@ Table *table_create(char kind, const GridDesc g[3], int num_splines, int storage
     all.insert(all.end(), one.begin(), one.end());
   }
   t->fast_solve = fast_solve_fits(t);
+  order_scratch_init(t);
   if (cudaMalloc(&t->factors_d, all.size() * sizeof(double)) != cudaSuccess ||
       cudaMemcpy(t->factors_d, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
     cudaGetLastError();
@@ -555,6 +556,7 @@ void table_destroy(Table *t) {
   if (t->wait_err_h) cudaFreeHost(t->wait_err_h);
   cudaFree(t->pipe_dev);
   cudaFree(t->sort_dev);
+  order_scratch_free(t);
   for (int i = 0; i < 2; i++) {
     if (t->pipe_stream[i]) cudaStreamDestroy(t->pipe_stream[i]);
     if (t->pipe_event[i]) cudaEventDestroy(t->pipe_event[i]);

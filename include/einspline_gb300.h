@@ -133,7 +133,12 @@ typedef struct {
   int sort;       /* 1: visit points in cell (Morton) order for L2 reuse; the
                      results are bit-identical to sort = 0.  The ordering
                      uses the table's sort scratch: sorted calls on one
-                     table on different streams must not overlap          */
+                     table on different streams must not overlap.
+                     0: the library decides: large batches on tables above
+                     192 MB go in cell order too, in scratch made with the
+                     table (7 MB) and from any number of streams at once;
+                     others, and launches under stream capture, keep
+                     their order.  The *_cuda entries do the same          */
   int64_t vstride, gstride, hstride; /* per-point output strides in output
                      reals (float for s/c, double for d/z); 0 = packed       */
 } einspline_gb300_eval_opts;
