@@ -333,6 +333,7 @@ int launch_eval_ordered(Table *t, EvalArgs &a, bool vgh, cudaStream_t s) {
   int tx, ty, pb;
   auto plain = [&]() {
     pick_tile(t, vgh, a.npts, tx, ty, pb);
+    fit_tile(t, a, vgh, tx, ty, pb);
     return launch_eval(t, a, vgh, s, tx, ty, pb);
   };
   if (!order_pays(t, a, vgh)) return plain();
@@ -372,6 +373,7 @@ int launch_eval_ordered(Table *t, EvalArgs &a, bool vgh, cudaStream_t s) {
     if (r) break;
     a.perm = perm;
     pick_tile(t, vgh, a.npts, tx, ty, pb, true);
+    fit_tile(t, a, vgh, tx, ty, pb);
     r = launch_eval(t, a, vgh, s, tx, ty, pb);
   }
   const cudaError_t e = cudaEventRecord(sl.done, s);
@@ -417,7 +419,8 @@ static int eval_device(Table *t, const einspline_gb300_eval_opts *o, int64_t npt
   if (int r = sort_points(t, a, &perm, s)) return r;
   a.perm = perm;
   int tx, ty, pb;
-  pick_tile(t, o->vgh != 0, npts, tx, ty, pb, a.perm != nullptr);
+  pick_tile(t, o->vgh != 0, npts, tx, ty, pb, true);
+  fit_tile(t, a, o->vgh != 0, tx, ty, pb);
   return launch_eval(t, a, o->vgh != 0, s, tx, ty, pb);
 }
 

@@ -277,6 +277,8 @@ int prepare_eval(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb, const 
 // sorted: the launch visits its points in cell order (a visiting order is
 // set), which has its own tuned shape.
 void pick_tile(Table *t, bool vgh, int64_t npts, int &tx, int &ty, int &pb, bool sorted = false);
+// Shrinks a picked tile for a batch (a.npts, a.perm) that would leave SMs idle.
+void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb);
 // Load mode of launches on this table (see EvalArgs::mode).
 int pick_mode(Table *t, bool vgh, bool sorted = false);
 // Tensor map of a 16-bit table for the tensor-core kernels (load mode 5).

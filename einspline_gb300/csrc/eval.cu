@@ -18,6 +18,7 @@
 #include <limits.h>
 #include <string.h>
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -1067,10 +1068,20 @@ static size_t max_smem_optin() {
   return (size_t)v;
 }
 
-// Kernel, block and dynamic shared memory of a launch; the pipelined kernels
-// run one point lane (ty = 1) and need their stage buffers raised above the
-// 48 KB default once per kernel.
-static int shape_launch(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb, const void **func, dim3 *block,
+// Stage buffers above the 48 KB default have to be allowed for a kernel, also
+// before its occupancy is asked for.
+static int raise_smem(const void *func, size_t smem) {
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return cuda_check(e, "cudaFuncSetAttribute(max dynamic shared memory)");
+  }
+  return 0;
+}
+
+// Kernel, block and dynamic shared memory of a launch, and a.pb, a.mode,
+// a.ntiles, a.coefs and a.box_bytes; the pipelined kernels run one point
+// lane (ty = 1).
+static int shape_kernel(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb, const void **func, dim3 *block,
                         size_t *smem, int mode = -1) {
   if (tx < 32 || tx % 32 || ty < 1 || tx * ty > 256 || pb < 1 || pb > 64)
     return fail(EINSPLINE_GB300_EINVAL, "bad launch shape tx=%d ty=%d pb=%d", tx, ty, pb);
@@ -1095,8 +1106,6 @@ static int shape_launch(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb,
     tx = kTcThreads;
     ty = 1;
     a.ntiles = (a.ncol + kTcCols - 1) / kTcCols;
-    a.wait_err = t->wait_err_d;
-    if (int r = tc_table_map(t, a)) return r;
     *smem = tc_smem(pb);
   } else if (a.mode == 4) {
     ty = 1;
@@ -1106,8 +1115,6 @@ static int shape_launch(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb,
     a.ntiles = (a.ncol + tx * VW - 1) / (tx * VW);
     const int es = is16(t->storage) ? 2 : (ks == ST_F32 ? 4 : 8);
     a.box_bytes = tx * 16 < 256 * es ? tx * 16 : 256 * es;
-    a.wait_err = t->wait_err_d;
-    if (int r = encode_table_map(t, a.coefs, es, a.box_bytes / es, &a.tmap)) return r;
     *smem = tma_smem(pb, acc_bytes(t), tx, stages);
   } else if (a.mode >= 2) {
     ty = 1;
@@ -1123,11 +1130,19 @@ static int shape_launch(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb,
     case ST_I16: *func = vgh ? kernel_for<ST_I16, true>(a.mode) : kernel_for<ST_I16, false>(a.mode); break;
     default: *func = vgh ? kernel_for<ST_F64, true>(a.mode) : kernel_for<ST_F64, false>(a.mode); break;
   }
-  if (*smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(*func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem);
-    if (e != cudaSuccess) return cuda_check(e, "cudaFuncSetAttribute(max dynamic shared memory)");
-  }
   return 0;
+}
+
+// The same ready to launch, with the tensor map of the modes that take one.
+static int shape_launch(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb, const void **func, dim3 *block,
+                        size_t *smem, int mode = -1) {
+  if (int r = shape_kernel(t, a, vgh, tx, ty, pb, func, block, smem, mode)) return r;
+  if (a.mode >= 4) {
+    a.wait_err = t->wait_err_d;
+    const int es = is16(t->storage) ? 2 : (kernel_storage(t) == ST_F32 ? 4 : 8);
+    if (int r = a.mode == 5 ? tc_table_map(t, a) : encode_table_map(t, a.coefs, es, a.box_bytes / es, &a.tmap)) return r;
+  }
+  return raise_smem(*func, *smem);
 }
 
 // Blocks of a kernel that one SM holds at once, looked up once per
@@ -1158,11 +1173,89 @@ static int resident_blocks(const void *func, int threads, size_t smem) {
   return cache[k] = per_sm * sms;
 }
 
+static int num_sms() {
+  static std::mutex mu;
+  static std::map<int, int> cache;
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return 152; }
+  std::lock_guard<std::mutex> g(mu);
+  auto it = cache.find(dev);
+  if (it != cache.end()) return it->second;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) { cudaGetLastError(); return 152; }
+  return cache[dev] = n;
+}
+
+// Smaller blocks for a batch that does not fill the GPU with the given
+// ones.  A block goes through its points one after another, so a batch of
+// 48 points in blocks of 8 or 10 left most SMs idle for 8 or 10 points'
+// time.  Among the shapes whose blocks are all resident at once, the one with
+// the least work on the fullest SM (points x columns), then the shortest
+// chain of points in a block; shapes with the same columns a block before
+// narrower ones.  Results do not depend on the shape.
+//
+// Measured, kernel time in us, given shape / this rule's / best of a scan
+// (vgh):
+//             F32 64^3 x 1024    F16 64^3 x 1024    I16 64^3 x 512     F32 45^3 x 203
+//   8 points  17.1 / 3.8 / 3.8    9.1 / 4.1 / 4.1   27.1 / 5.3 / 5.3   18.5 / 3.9 / 3.9
+//   48        17.4 / 5.0 / 5.0   10.6 / 5.3 / 4.9   27.2 / 5.4 / 5.4   18.5 / 4.0 / 4.0
+//   300       18.2 / 13.9 / 13.6 10.8 / 9.3 / 8.8   27.5 / 8.0 / 8.0   18.8 / 6.6 / 6.6
+//   1000      53.1 / 53 / 51     29.0 / 29 / 29     31.6 / 18.9 / 18.9 18.9 / 14.7 / 14.5
+//   3000      unchanged          unchanged          52.1 / 45 / 44     34.4 / 32 / 32
+// A batch of at least one full wave keeps the shape, as do shapes set by
+// set_tile.
+void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) {
+  if (t->tile_tx || a.npts <= 0) return;
+  EvalArgs b = a;
+  const void *func;
+  dim3 block;
+  size_t smem;
+  if (shape_kernel(t, b, vgh, tx, ty, pb, &func, &block, &smem) || raise_smem(func, smem)) return;
+  const int64_t sms = num_sms();
+  // (the occupancy query answers 1 for kernels that allocate tensor memory;
+  // kTcBlocksPerSM of theirs fit)
+  const int64_t wave = b.mode == 5 ? kTcBlocksPerSM * sms : resident_blocks(func, (int)(block.x * block.y), smem);
+  const int64_t per = wave / sms;
+  if (per < 1) return;
+  // Direct loads hide their latency only behind other warps, and their
+  // blocks start quickly: one point a lane below four waves of the given
+  // blocks (FP32 values, 40^3 x 1000, 3000 points: 86 against 99 us; from
+  // five waves on, 4 points a lane are up to 10 % faster), for FP64, which its
+  // arithmetic bounds, below one.
+  if (b.mode == 0 && (a.npts + pb - 1) / pb * b.ntiles < (t->storage == ST_F64 ? 1 : 4) * wave) pb = (int)block.y;
+  if ((a.npts + pb - 1) / pb * b.ntiles >= wave) return;
+  // modes 3 and 5 have one block width; the others' blocks narrow by halves
+  const bool fixed = b.mode == 3 || b.mode == 5;
+  const int width = fixed ? tx : (int)block.x, lanes = (int)block.y;
+  int best[3] = {tx, ty, pb};
+  int64_t best_work = INT64_MAX, best_chain = 0;
+  for (int x = width; x >= 32; x = x > 32 ? (x / 2 + 31) / 32 * 32 : 0) {
+    if (fixed && x != width) break;
+    const int64_t tiles = fixed ? b.ntiles : ((int64_t)b.ntiles * width + x - 1) / x;
+    for (int y = lanes; y >= 1; y /= 2) {
+      const int64_t fit = fixed ? per : std::min<int64_t>(32, per * width * lanes / (x * y));
+      for (int p = y; p <= pb; p += y) {
+        const int64_t blocks = (a.npts + p - 1) / p * tiles, deep = (blocks + sms - 1) / sms;
+        if (deep > fit) continue;
+        const int64_t work = deep * p * x, chain = p / y;
+        if (work < best_work || (work == best_work && chain < best_chain)) {
+          best_work = work;
+          best_chain = chain;
+          best[0] = x; best[1] = y; best[2] = p;
+        }
+      }
+    }
+  }
+  tx = best[0]; ty = best[1]; pb = best[2];
+}
+
 // Point groups of a launch.  A launch of more than two waves gives the
 // points of its last wave of full groups to groups of pb/4 points: every
 // block computes its points the same way whatever its group holds, so the
 // results do not change, and the launch ends with short blocks instead of
-// SMs idling while the last full ones finish.
+// SMs idling while the last full ones finish.  (For the tensor-core kernel a
+// wave here is one block an SM, the occupancy query's answer for kernels that
+// allocate tensor memory; its true three measured up to 10 % slower: too
+// many short blocks.)
 static int64_t plan_groups(EvalArgs &a, const void *func, dim3 block, size_t smem) {
   a.pb_tail = 0;
   a.g_tail = 0;
@@ -1279,6 +1372,23 @@ void pick_tile(Table *t, bool vgh, int64_t npts, int &tx, int &ty, int &pb, bool
     tx = tx > cap ? cap : tx;
     ty = 1;
     pb = 8;
+    return;
+  }
+  // Direct loads.  IEEE FP64 vgh: blocks of 128 threads with 4 points a lane
+  // (48^3 x 512, 8192 points: 2331 us; 256 threads with 2 points 2435);
+  // FP32 values: 64 threads with 4 points (45^3 x 203, 20,000 points: 69.5
+  // against 77.4 us for 64 x 4 threads with 2 points a lane; 40^3 x 512: 192
+  // against 200).
+  if (kernel_storage(t) == ST_F64 && vgh) {
+    if (tx > 128) tx = 128;
+    ty = std::min(8, 128 / tx);
+    pb = 4 * ty;
+    return;
+  }
+  if (!vgh && t->storage == ST_F32 && t->tile_mode <= 0) {
+    if (tx > 64) tx = 64;
+    ty = 1;
+    pb = 4;
     return;
   }
   if (tx > 256) tx = 256;

@@ -674,6 +674,7 @@ constexpr int kTcCols = 128 * kTcTiles;  // columns per block
 constexpr int kTcN = 32;                 // 10 outputs x weight parts (<= 3), padded to the MMA's N
 constexpr int kTcThreads = 192;          // copy warp, MMA warp, 4 weight/output warps
 constexpr int kTcStages = 4;             // stencil stages, one 128-column tile of a point each
+constexpr int kTcBlocksPerSM = 3;        // by shared memory, up to 11 points a block
 // Per table type: an FP32 weight is the sum of two f16 parts (22 bits) or of
 // three bf16 parts (exactly: 3 x 8 bits), each part accumulating in its own
 // column, summed in the epilogue.

@@ -186,6 +186,7 @@ extern "C" int einspline_gb300_eval_3d_sorted_noalloc(einspline_gb300_table *t, 
     int *perm = nullptr;
     if (int r = small_sort_into(a, scratch, &perm, s)) return r;
     a.perm = perm;
+    fit_tile(t, a, o->vgh != 0, tx, ty, pb);
     return launch_eval(t, a, o->vgh != 0, s, tx, ty, pb);
   }
   char *p = (char *)scratch;

@@ -240,12 +240,14 @@ static int launch_batch(Server *v, Slot &s) {
   const int64_t n = s.points;
   EvalArgs a;
   fill_args(v, s, a, n);
+  int tx = v->tx, ty = v->ty, pb = v->pb;
   const size_t bytes = (size_t)n * (24 + v->pos_b);
   if (v->o.use_graphs) {
     const void *func;
     dim3 grid, block;
     size_t smem;
-    if (int r = prepare_eval(v->t, a, v->o.vgh != 0, v->tx, v->ty, v->pb, &func, &grid, &block, &smem)) return r;
+    fit_tile(v->t, a, v->o.vgh != 0, tx, ty, pb);
+    if (int r = prepare_eval(v->t, a, v->o.vgh != 0, tx, ty, pb, &func, &grid, &block, &smem)) return r;
     cudaKernelNodeParams kp;
     memset(&kp, 0, sizeof(kp));
     void *args[] = {&a};
@@ -265,7 +267,8 @@ static int launch_batch(Server *v, Slot &s) {
       if (int r = small_sort_into(a, s.sort_d, &perm, s.stream)) return r;
       a.perm = perm;
     }
-    if (int r = launch_eval(v->t, a, v->o.vgh != 0, s.stream, v->tx, v->ty, v->pb)) return r;
+    fit_tile(v->t, a, v->o.vgh != 0, tx, ty, pb);
+    if (int r = launch_eval(v->t, a, v->o.vgh != 0, s.stream, tx, ty, pb)) return r;
     EG_CUDA(cudaEventRecord(s.done, s.stream));
   }
   return 0;
