@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kDetThreads, kDetBlocksPerSM) k_det_ratio(cons
 // Two stencil stages and five blocks an SM: more walkers in flight than four
 // stages and three blocks (2,048 walkers: 0.047 against 0.052 ms; 16,384:
 // 0.285 against 0.298 ms).
-constexpr int kDtStages = 2, kDtSlots = 4, kDtMaxWalkers = 7, kDtBlocksPerSM = 5;
+constexpr int kDtStages = 2, kDtSlots = 4, kDtMaxWalkers = 7, kDtBlocksPerSM = 5, kDtUnits = 8;
 __host__ __device__ __forceinline__ size_t dt_ptr_off(int pb) { return align_up(smem_total(pb, 4), 16); }
 __host__ __device__ __forceinline__ size_t dt_red_off(int pb) { return dt_ptr_off(pb) + (size_t)pb * 8; }
 __host__ __device__ __forceinline__ size_t dt_head(int pb) { return dt_red_off(pb) + (size_t)pb * 4 * 5 * 4; }
@@ -1173,17 +1173,25 @@ int einspline_gb300_det_ratio(einspline_gb300_table *t, const einspline_gb300_de
   const bool gl = grad_d || lapl_d;
   cudaStream_t s = stream ? (cudaStream_t)stream : cudaStreamLegacy;
   if ((t->storage == ST_F16 || t->storage == ST_BF16) && pick_mode(t, true) == 5) {
-    // tensor cores, as the table's vgh evaluation: kDtBlocksPerSM blocks of at most
-    // kDtMaxWalkers walkers an SM, the walkers spread evenly over whole waves
+    // tensor cores, as the table's vgh evaluation
     if (int r = tc_table_map(t, d.e)) return r;
     d.e.wait_err = t->wait_err_d;
     if (t->test_skip.load(std::memory_order_relaxed)) {
       d.e.test_skip = t->test_skip.exchange(0);
       d.e.wait_ns = t->test_wait_ns;
     }
-    const int64_t slots = kDtBlocksPerSM * (int64_t)num_sms();
-    const int64_t waves = (nwalkers + slots * kDtMaxWalkers - 1) / (slots * kDtMaxWalkers);
-    const int pb = (int)((nwalkers + slots * waves - 1) / (slots * waves));
+    // Blocks of about kDtUnits tiles: long enough for the copies to run ahead
+    // of a block's set-up, short enough for the last wave to end evenly;
+    // beyond four waves of them, longer ones.  us
+    // a ratio with gradient and laplacian, walkers spread over whole waves
+    // of at most 7 a block (before) / this: N = 1024, 2048 walkers 99.4 / 95.6
+    // (transposed inverse 49.5 / 47.6), 4096 walkers 186 / 179 (88.5 /
+    // 85.1); N = 256, 4096 walkers 52 / 50 (26.8 / 24.7).  Bound by DRAM's
+    // random reads: the stencils and, in the reference's layout, 128 bytes
+    // for each inverse entry.
+    const int tiles = (d.n + 127) / 128;
+    const int64_t wave = kDtBlocksPerSM * (int64_t)num_sms();
+    const int pb = (int)std::min<int64_t>(kDtMaxWalkers, std::max<int64_t>(std::max(1, kDtUnits / tiles), nwalkers / (4 * wave)));
     d.e.pb = pb;
     const unsigned grid = (unsigned)((nwalkers + pb - 1) / pb);
     EG_CUDA(t->storage == ST_F16 ? launch_det_tc<ST_F16>(d, gl, grid, s) : launch_det_tc<ST_BF16>(d, gl, grid, s));
