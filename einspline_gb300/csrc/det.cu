@@ -1063,9 +1063,8 @@ cudaLaunchConfig_t cluster_config(int blocks, int cs, int threads, size_t smem, 
 }
 
 // Clusters of a kernel that the current device holds at once (0: none, or
-// the query failed), looked up once per kernel, shape and device; the
-// kernel's shared-memory limit is raised to most, its largest launch's.
-int resident_clusters(const void *func, int cs, int threads, size_t smem, size_t most) {
+// the query failed), looked up once per kernel, shape and device.
+int resident_clusters(const void *func, int cs, int threads, size_t smem) {
   struct Key {
     const void *f;
     int cs, threads, dev;
@@ -1085,9 +1084,8 @@ int resident_clusters(const void *func, int cs, int threads, size_t smem, size_t
   int fit = 0;
   cudaLaunchAttribute at;
   const cudaLaunchConfig_t lc = cluster_config(cs, cs, threads, smem, nullptr, &at);
-  if ((most > 48 * 1024 &&
-       cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) ||
-      cudaOccupancyMaxActiveClusters(&fit, func, &lc) != cudaSuccess) {
+  if (allow_smem(func, smem)) return 0;
+  if (cudaOccupancyMaxActiveClusters(&fit, func, &lc) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
@@ -1110,8 +1108,7 @@ cudaError_t launch_ratio_k(const DetArgs &d, unsigned grid, cudaStream_t s) {
   constexpr int RB = WIDE ? 16 : (int)sizeof(typename CT<ST>::Raw);
   const size_t sm = det_smem(d.e.pb, RB);
   const void *f = (const void *)k_det_ratio<ST, GL, WIDE>;
-  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return e;
+  if (allow_smem(f, sm)) return cudaErrorInvalidValue;
   k_det_ratio<ST, GL, WIDE><<<grid, kDetThreads, sm, s>>>(d);
   return cudaGetLastError();
 }
@@ -1125,8 +1122,7 @@ template <int ST, bool GL>
 cudaError_t launch_det_tc_k(const DetArgs &d, unsigned grid, cudaStream_t s) {
   const size_t sm = dt_smem(d.e.pb);
   const void *f = (const void *)k_det_tc<ST, GL>;
-  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-  if (e != cudaSuccess) return e;
+  if (allow_smem(f, sm)) return cudaErrorInvalidValue;
   k_det_tc<ST, GL><<<grid, kTcThreads, sm, s>>>(d);
   return cudaGetLastError();
 }
@@ -1245,8 +1241,7 @@ int einspline_gb300_det_update(const einspline_gb300_det_opts *o, int naccept, f
     const void *f = sh.threads == 128 ? update_kernel<128>(d.trans)
                   : sh.threads == 256 ? update_kernel<256>(d.trans) : update_kernel<512>(d.trans);
     const size_t sm = up_smem(d.n, sh.cs, d.trans, sh.threads);
-    const size_t most = up_smem(std::min(kUpMax, kUpVec * sh.threads), sh.cs, d.trans, sh.threads);
-    const int fit = resident_clusters(f, sh.cs, sh.threads, sm, most);
+    const int fit = resident_clusters(f, sh.cs, sh.threads, sm);
     if (fit > 0) {
       const int clusters = std::min(naccept, fit);
       int lpr_log = 0;

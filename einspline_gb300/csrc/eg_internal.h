@@ -260,6 +260,10 @@ struct EvalArgs {
   CUtensorMap tmap;
 };
 
+// Largest dynamic shared memory a block may opt into on the current device,
+// and leave for a kernel to be launched with (or asked about at) smem bytes.
+size_t max_smem_optin();
+int allow_smem(const void *func, size_t smem);
 // mode >= 0 forces a load mode (EvalArgs::mode) instead of the table's choice.
 int launch_eval(Table *t, EvalArgs &a, bool vgh, cudaStream_t s, int tx, int ty, int pb, int mode = -1);
 // One point of a single-point entry (a.npts = 1, outputs in the point scratch).

@@ -1058,7 +1058,7 @@ int tc_table_map(const Table *t, EvalArgs &a) {
 }
 
 // Largest dynamic shared memory a block may opt into on the current device.
-static size_t max_smem_optin() {
+size_t max_smem_optin() {
   int dev = 0, v = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
@@ -1068,14 +1068,12 @@ static size_t max_smem_optin() {
   return (size_t)v;
 }
 
-// Stage buffers above the 48 KB default have to be allowed for a kernel, also
-// before its occupancy is asked for.
-static int raise_smem(const void *func, size_t smem) {
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_check(e, "cudaFuncSetAttribute(max dynamic shared memory)");
-  }
-  return 0;
+// A kernel's limit is always raised to the device's largest, so that threads
+// launching it with different sizes do not lower it for each other.
+int allow_smem(const void *func, size_t smem) {
+  if (smem <= 48 * 1024) return 0;
+  const cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem_optin());
+  return e == cudaSuccess ? 0 : cuda_check(e, "cudaFuncSetAttribute(max dynamic shared memory)");
 }
 
 // Kernel, block and dynamic shared memory of a launch, and a.pb, a.mode,
@@ -1142,7 +1140,7 @@ static int shape_launch(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb,
     const int es = is16(t->storage) ? 2 : (kernel_storage(t) == ST_F32 ? 4 : 8);
     if (int r = a.mode == 5 ? tc_table_map(t, a) : encode_table_map(t, a.coefs, es, a.box_bytes / es, &a.tmap)) return r;
   }
-  return raise_smem(*func, *smem);
+  return allow_smem(*func, *smem);
 }
 
 // Blocks of a kernel that one SM holds at once, looked up once per
@@ -1209,7 +1207,7 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   const void *func;
   dim3 block;
   size_t smem;
-  if (shape_kernel(t, b, vgh, tx, ty, pb, &func, &block, &smem) || raise_smem(func, smem)) return;
+  if (shape_kernel(t, b, vgh, tx, ty, pb, &func, &block, &smem) || allow_smem(func, smem)) return;
   const int64_t sms = num_sms();
   // (the occupancy query answers 1 for kernels that allocate tensor memory;
   // kTcBlocksPerSM of theirs fit)

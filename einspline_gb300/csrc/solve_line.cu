@@ -293,11 +293,6 @@ __global__ void __launch_bounds__(32) k_solve_z(const FastArgs a) {
 // 64-row lines share an SM's shared memory.
 constexpr int kLines = 32;
 
-int raise_smem(const void *f, size_t bytes) {
-  if (bytes > 48 * 1024) EG_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  return 0;
-}
-
 }  // namespace
 
 void pack_fast_factors(const LineFactors &f, std::vector<double> &out) {
@@ -378,12 +373,12 @@ int solve_fast(Table *t, int n, cudaStream_t s) {
   const unsigned gx = (unsigned)(yzt * ((ncw + CW - 1) / CW));
   const void *fx = nc == 1 ? (const void *)k_solve_x<1> : (const void *)k_solve_x<2>;
   void *args[] = {&a};
-  if (int r = raise_smem(fx, sm)) return r;
+  if (int r = allow_smem(fx, sm)) return r;
   EG_CUDA(cudaLaunchKernel(fx, dim3(gx), dim3(CW * YZ), args, sm, s));
   // y
   axis(1);
   sm = (size_t)kLines * a.My * sizeof(double);
-  if (int r = raise_smem((const void *)k_solve_y, sm)) return r;
+  if (int r = allow_smem((const void *)k_solve_y, sm)) return r;
   k_solve_y<<<dim3((unsigned)(((int64_t)a.Mz * ncw + kLines - 1) / kLines), (unsigned)Nx), kLines, sm, s>>>(a);
   EG_CUDA(cudaGetLastError());
   // z
@@ -395,7 +390,7 @@ int solve_fast(Table *t, int n, cudaStream_t s) {
   a.slot_spline = t->slot_spline_d;
   a.colmax = (unsigned *)t->colmax;
   if (!a.table) EG_CUDA(cudaMemsetAsync(t->colmax, 0, ncw * sizeof(unsigned), s));
-  if (int r = raise_smem((const void *)k_solve_z, sm)) return r;
+  if (int r = allow_smem((const void *)k_solve_z, sm)) return r;
   k_solve_z<<<(unsigned)((a.nlines * ncw + kLines - 1) / kLines), kLines, sm, s>>>(a);
   EG_CUDA(cudaGetLastError());
   count_launch(3);
