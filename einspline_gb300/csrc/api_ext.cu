@@ -275,14 +275,16 @@ int sort_points(Table *t, const EvalArgs &a, int **perm_out, cudaStream_t s) {
 // Tables near the 129 MB L2 are mostly served by it in any order.  I16 vgh
 // is bound by its arithmetic, and FP64 tables by theirs: IEEE arithmetic
 // never gains, double-float only on values (154/135 at 0.58 GB).
-constexpr size_t kOrderTableBytes = 192u << 20;
-constexpr double kOrderSavedBytes = 0.5e9, kOrderSavedBytesI16 = 2e9;
+// Where L2 holds a good part of the table more has to be saved.
+constexpr size_t kOrderTableBytes = 192u << 20, kOrderLargeTable = 512u << 20;
+constexpr double kOrderSavedBytes = 0.5e9, kOrderSavedLarge = 0.3e9, kOrderSavedBytesI16 = 2e9;
 
 static bool order_pays(const Table *t, const EvalArgs &a, bool vgh) {
   if (!t->order_dev || (t->storage == ST_F64 && (vgh || t->fp64_mode != 1))) return false;
   const double R = (double)t->Nc[0] * t->Nc[1] * t->Nc[2], n64 = 64.0 * (double)a.npts;
   const double saved = (n64 - R * (1.0 - exp(-n64 / R))) * (double)t->zs * t->elem_bytes;
-  return saved > (vgh && t->storage == ST_I16 ? kOrderSavedBytesI16 : kOrderSavedBytes);
+  return saved > (vgh && t->storage == ST_I16 ? kOrderSavedBytesI16
+                  : t->table_bytes >= kOrderLargeTable ? kOrderSavedLarge : kOrderSavedBytes);
 }
 
 void order_scratch_init(Table *t) {
@@ -631,7 +633,7 @@ int einspline_gb300_set_tile(einspline_gb300_table *t, int tx, int ty, int pb) {
 int einspline_gb300_get_tile(einspline_gb300_table *t, int *tx, int *ty, int *pb) {
   clear();
   if (!table3_ok(t) || !tx || !ty || !pb) return fail(EINSPLINE_GB300_EINVAL, "bad argument");
-  pick_tile(t, true, 0, *tx, *ty, *pb);
+  pick_tile(t, true, 1, *tx, *ty, *pb);
   return 0;
 }
 
@@ -639,7 +641,7 @@ int einspline_gb300_get_launch_shape(einspline_gb300_table *t, int sorted, int v
                                      int *mode) {
   clear();
   if (!table3_ok(t) || !tx || !ty || !pb || !mode) return fail(EINSPLINE_GB300_EINVAL, "bad argument");
-  pick_tile(t, vgh != 0, 0, *tx, *ty, *pb, sorted != 0);
+  pick_tile(t, vgh != 0, 1, *tx, *ty, *pb, sorted != 0);
   *mode = pick_mode(t, vgh != 0, sorted != 0);
   return 0;
 }

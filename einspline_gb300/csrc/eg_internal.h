@@ -284,7 +284,7 @@ void pick_tile(Table *t, bool vgh, int64_t npts, int &tx, int &ty, int &pb, bool
 // Shrinks a picked tile for a batch (a.npts, a.perm) that would leave SMs idle.
 void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb);
 // Load mode of launches on this table (see EvalArgs::mode).
-int pick_mode(Table *t, bool vgh, bool sorted = false);
+int pick_mode(Table *t, bool vgh, bool sorted = false, int64_t npts = 1);
 // Tensor map of a 16-bit table for the tensor-core kernels (load mode 5).
 int tc_table_map(const Table *t, EvalArgs &a);
 int elems_per_thread(const Table *t);

@@ -16,6 +16,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <limits.h>
+#include <math.h>
 #include <string.h>
 
 #include <algorithm>
@@ -1084,7 +1085,7 @@ static int shape_kernel(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb,
   if (tx < 32 || tx % 32 || ty < 1 || tx * ty > 256 || pb < 1 || pb > 64)
     return fail(EINSPLINE_GB300_EINVAL, "bad launch shape tx=%d ty=%d pb=%d", tx, ty, pb);
   a.pb = pb;
-  a.mode = mode >= 0 ? mode : pick_mode(t, vgh, a.perm != nullptr);
+  a.mode = mode >= 0 ? mode : pick_mode(t, vgh, a.perm != nullptr, a.npts);
   const int ks = kernel_storage(t);
   if (a.mode >= 2 && ks == ST_F64) a.mode = 0;        // IEEE FP64 is FMA-bound: no pipeline variant
   // tensor cores: F16 and BF16 tables; one column a thread, so not the
@@ -1214,13 +1215,28 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   const int64_t wave = b.mode == 5 ? kTcBlocksPerSM * sms : resident_blocks(func, (int)(block.x * block.y), smem);
   const int64_t per = wave / sms;
   if (per < 1) return;
-  // Direct loads hide their latency only behind other warps, and their
-  // blocks start quickly: one point a lane below four waves of the given
-  // blocks (FP32 values, 40^3 x 1000, 3000 points: 86 against 99 us; from
-  // five waves on, 4 points a lane are up to 10 % faster), for FP64, which its
+  // Values by direct loads hide their latency only behind other warps, and
+  // their blocks start quickly: one point a lane below four waves of the given
+  // blocks (FP32, 40^3 x 1000, 3000 points: 86 against 99 us; from five
+  // waves on, 4 points a lane are up to 10 % faster), for FP64, which its
   // arithmetic bounds, below one.
-  if (b.mode == 0 && (a.npts + pb - 1) / pb * b.ntiles < (t->storage == ST_F64 ? 1 : 4) * wave) pb = (int)block.y;
-  if ((a.npts + pb - 1) / pb * b.ntiles >= wave) return;
+  if (b.mode == 0 && (!vgh || t->storage == ST_F64) && (a.npts + pb - 1) / pb * b.ntiles < (t->storage == ST_F64 ? 1 : 4) * wave) pb = (int)block.y;
+  const int64_t full = (a.npts + pb - 1) / pb * b.ntiles;
+  if (full >= wave) {
+    // between one and two waves of the copy pipelines' blocks: the size whose
+    // whole waves take the least points one after another (FP32 48^3 x 400,
+    // 3001 points vgl: 51.4 us with 5 points a block, 57.5 with 8)
+    if (b.mode < 2 || b.mode > 4 || full > 2 * wave) return;
+    int64_t best = INT64_MAX;
+    for (int p = pb, p0 = pb; p >= (p0 + 1) / 2; p--) {
+      const int64_t cost = ((a.npts + p - 1) / p * b.ntiles + wave - 1) / wave * p;
+      if (cost < best) {
+        best = cost;
+        pb = p;
+      }
+    }
+    return;
+  }
   // modes 3 and 5 have one block width; the others' blocks narrow by halves
   const bool fixed = b.mode == 3 || b.mode == 5;
   const int width = fixed ? tx : (int)block.x, lanes = (int)block.y;
@@ -1305,14 +1321,18 @@ int load_eval_kernel(Table *t, bool vgh, bool sorted) {
   fill_eval_geometry(t, a);
   static const int one = 0;
   if (sorted) a.perm = &one;  // only its presence matters: it selects the sorted launch shape
-  int tx, ty, pb;
-  pick_tile(t, vgh, 1, tx, ty, pb, sorted);
-  const void *func;
-  dim3 block;
-  size_t smem;
-  if (int r = shape_launch(t, a, vgh, tx, ty, pb, &func, &block, &smem)) return r;
-  cudaFuncAttributes fa;
-  EG_CUDA(cudaFuncGetAttributes(&fa, func));
+  // the choice may depend on the batch size: few points and many
+  for (int64_t n : {(int64_t)1, (int64_t)1 << 40}) {
+    int tx, ty, pb;
+    a.npts = n;
+    pick_tile(t, vgh, n, tx, ty, pb, sorted);
+    const void *func;
+    dim3 block;
+    size_t smem;
+    if (int r = shape_launch(t, a, vgh, tx, ty, pb, &func, &block, &smem)) return r;
+    cudaFuncAttributes fa;
+    EG_CUDA(cudaFuncGetAttributes(&fa, func));
+  }
   return 0;
 }
 
@@ -1330,7 +1350,32 @@ int prepare_eval(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb, const 
 // copy pipeline, 8-column wide for 16-bit tables; value-only evaluation uses
 // the wide pipeline for 16-bit tables and direct loads otherwise; IEEE FP64
 // (FMA-bound) always uses direct loads.
-int pick_mode(Table *t, bool vgh, bool sorted) {
+// Points per stencil row that npts uniform points touch.
+static double row_reuse(const Table *t, int64_t npts) {
+  const double R = (double)t->Nc[0] * t->Nc[1] * t->Nc[2], n64 = 64.0 * (double)std::max<int64_t>(npts, 1);
+  return n64 / (R * (1.0 - exp(-n64 / R)));
+}
+
+// FP32 vgh by direct loads instead of the copy pipeline.  The pipeline's
+// copies bypass L1; they win where rows come from DRAM.  Direct loads
+// win where rows come from L2, and from L1 when a block's points share them:
+// tables that L2 holds, and launches in cell order once rows are shared
+// enough.  us a launch, pipeline / direct (32 x 2 or 4 threads, 4 points a
+// lane):
+//   random order   45^3 x 203 (97 MB) 8000 points      79 / 63
+//                  30^3 x 256 (37 MB) 30,000           193 / 148
+//                  48^3 x 512 (271 MB) 8000            135 / 141
+//   cell order     48^3 x 512 4000 (2.3 a row)         72 / 64
+//                  64^3 x 1024 12,000 (2.8)            328 / 335
+//                  64^3 x 256 complex 16,384 (3.6)     219 / 208
+//                  64^3 x 1024 60,000 (13)             1521 / 1230
+constexpr size_t kL2Table = 112u << 20, kNearL2Table = 300u << 20;
+static bool direct_pays(const Table *t, bool sorted, int64_t npts) {
+  if (t->table_bytes < kL2Table) return true;
+  return sorted && (t->table_bytes < kNearL2Table || row_reuse(t, npts) >= 3.0);
+}
+
+int pick_mode(Table *t, bool vgh, bool sorted, int64_t npts) {
   if (t->tile_mode >= 0) return t->tile_mode;
   const int v = vgh ? 1 : 0;
   if (sorted && t->tuned_s_tx[v]) return t->tuned_s_mode[v];
@@ -1341,7 +1386,10 @@ int pick_mode(Table *t, bool vgh, bool sorted) {
   // and 46.1 G); value only stays on the wide pipeline (58.4 G random and
   // 90.9 G sorted against 57.8 G and 74.0 G for F16)
   if (vgh && (t->storage == ST_F16 || t->storage == ST_BF16)) return 5;
-  if (vgh && kernel_storage(t) != ST_F64) return is16(t->storage) ? 3 : 2;
+  if (vgh && kernel_storage(t) != ST_F64) {
+    if (is16(t->storage)) return 3;
+    return kernel_storage(t) == ST_F32 && direct_pays(t, sorted, npts) ? 0 : 2;
+  }
   // value only: the wide pipeline for 16-bit tables (0.294 against 0.413 ms
   // with direct loads at 64^3 x 1024, 17k points); FP32 is as fast direct
   if (is16(t->storage)) return 3;
@@ -1364,6 +1412,13 @@ void pick_tile(Table *t, bool vgh, int64_t npts, int &tx, int &ty, int &pb, bool
   const int VW = elems_per_thread(t);
   const int need = (t->ncol + VW - 1) / VW;
   tx = (need + 31) / 32 * 32;
+  if (vgh && kernel_storage(t) == ST_F32 && t->tile_mode <= 0 && (t->tile_mode == 0 || direct_pays(t, sorted, npts))) {
+    // in cell order more points share a block's L1
+    tx = 32;
+    ty = sorted ? 4 : 2;
+    pb = 4 * ty;
+    return;
+  }
   if ((vgh || is16(t->storage)) && kernel_storage(t) != ST_F64 && t->tile_mode < 0) {
     // pipelined defaults (pick_mode): one lane of points, 8 points a block
     const int cap = is16(t->storage) ? 32 : (kernel_storage(t) == ST_DF ? 128 : 64);
@@ -1373,10 +1428,11 @@ void pick_tile(Table *t, bool vgh, int64_t npts, int &tx, int &ty, int &pb, bool
     return;
   }
   // Direct loads.  IEEE FP64 vgh: blocks of 128 threads with 4 points a lane
-  // (48^3 x 512, 8192 points: 2331 us; 256 threads with 2 points 2435);
-  // FP32 values: 64 threads with 4 points (45^3 x 203, 20,000 points: 69.5
-  // against 77.4 us for 64 x 4 threads with 2 points a lane; 40^3 x 512: 192
-  // against 200).
+  // (48^3 x 512, 8192 points: 2331 us; 256 threads with 2 points 2435).  FP32
+  // values: one point a block of 64 threads; 4 points for tables that L2
+  // holds (45^3 x 203, 100,000 points: 279 against 303 us), 32 x 4 threads
+  // with 8 points where cell order shares rows (64^3 x 1024, 60,000 points:
+  // 638 against 717; 16,384 points: 266 against 257).
   if (kernel_storage(t) == ST_F64 && vgh) {
     if (tx > 128) tx = 128;
     ty = std::min(8, 128 / tx);
@@ -1384,16 +1440,16 @@ void pick_tile(Table *t, bool vgh, int64_t npts, int &tx, int &ty, int &pb, bool
     return;
   }
   if (!vgh && t->storage == ST_F32 && t->tile_mode <= 0) {
-    if (tx > 64) tx = 64;
-    ty = 1;
-    pb = 4;
+    const bool shared = sorted && row_reuse(t, npts) >= 4.5;
+    if (shared || tx > 64) tx = shared ? 32 : 64;
+    ty = shared ? 4 : 1;
+    pb = shared ? 8 : (!sorted && t->table_bytes < kL2Table) ? 4 : 1;
     return;
   }
   if (tx > 256) tx = 256;
   ty = 256 / tx;
   if (ty > 8) ty = 8;
   pb = 2 * ty;
-  (void)npts;
 }
 
 int wait_status(Table *t, const char *fn) {

@@ -216,9 +216,10 @@ int einspline_gb300_get_tile(einspline_gb300_table *t, int *tx, int *ty, int *pb
  *      points per block, so tuning changes no result.  Other tables, and
  *      complex tables in the CPU layout, use their pipeline (3 or 2) instead;
  *  -1: the autotuned choice; untuned, vgh uses 5 for F16 and BF16 tables, 3
- *      for I16 tables and 2 for FP32 (the choices the autotuner makes on
- *      GB300); value-only uses 3 for 16-bit tables and 0 for FP32; FP64
- *      uses 0.  Results are identical in modes 0-4, and within mode 5. */
+ *      for I16 tables, and for FP32 tables 2, or 0 where the stencil rows
+ *      come from L2 rather than memory (tables below 112 MB, and
+ *      launches in cell order that share rows enough); value-only uses 3
+ *      for 16-bit tables and 0 for FP32; FP64 uses 0.  Results are identical in modes 0-4, and within mode 5. */
 int einspline_gb300_set_load_mode(einspline_gb300_table *t, int mode);
 int einspline_gb300_get_load_mode(einspline_gb300_table *t);
 /* Every wait of the mode-4 and mode-5 kernels on their mbarriers is bounded (0.5 s);
