@@ -117,10 +117,12 @@ struct einspline_gb300_table {
   bool fast_solve = false;          // solved by solve_fast (fast_solve_fits)
   cudaStream_t stream = nullptr;
 
-  // single-point entry scratch: 40 * ncol output reals in mapped pinned
-  // host memory, which the kernels write directly
+  // single-point entry scratch: 40 * pt_cols(ncol) output reals in mapped
+  // pinned host memory, which the kernels write directly, then a word per
+  // block of k_point that holds the number of the last call it finished
   void *pt_host = nullptr;
   void *pt_dev = nullptr;           // its device address
+  unsigned pt_seq = 0;              // calls so far
 
   // host-buffer pipeline scratch (einspline_gb300_eval_3d_host)
   void *pipe_dev = nullptr;
@@ -266,12 +268,12 @@ size_t max_smem_optin();
 int allow_smem(const void *func, size_t smem);
 // mode >= 0 forces a load mode (EvalArgs::mode) instead of the table's choice.
 int launch_eval(Table *t, EvalArgs &a, bool vgh, cudaStream_t s, int tx, int ty, int pb, int mode = -1);
-// One point of a single-point entry (a.npts = 1, outputs in the point scratch).
-int launch_point(Table *t, EvalArgs &a, bool vgh);
 // ETIMEOUT (and clears the word) when a TMA-staged evaluation on t gave up a
 // bounded wait since the last check; call after the launches completed.
 int wait_status(Table *t, const char *fn);
-// Mapped pinned output scratch of the single-point entries (40 * ncol reals).
+// Mapped pinned output scratch of the single-point entries (40 * pt_cols(ncol)
+// reals; pt_cols rounds up so that each output array can start on 128 bytes).
+inline size_t pt_cols(int ncol) { return ((size_t)ncol + 31) / 32 * 32; }
 int point_scratch(Table *t, const char *fn);
 void fill_eval_geometry(const Table *t, EvalArgs &a);
 // Kernel, grid, block and shared memory of a launch without launching it

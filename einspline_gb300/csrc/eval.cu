@@ -20,6 +20,8 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <map>
 #include <mutex>
 #include <tuple>
@@ -1461,32 +1463,216 @@ int wait_status(Table *t, const char *fn) {
   return 0;
 }
 
-// Output scratch of the single-point entries: 40 output reals per column
-// (value, 3 gradient, 9 Hessian, 27 third-derivative) in pinned host memory
-// mapped into the device's address space.  The kernels write their outputs
-// there directly, so a call needs no device-to-host copy: after the stream
-// synchronises the host reads them in place.
+// ------------------------------------------------------------ single points
+// One point for the CPU-shaped entries (value, vg, vgl, vgh; CPU-entry cell
+// rule and CPU layouts).  A call is all latency, so the point is spread out:
+// a block owns 128 columns (32 of an FP64 table), each of its 4 warps reads
+// and reduces one x-plane of the stencil -- one round of 16 loads in flight
+// instead of four -- and the planes' y sums meet in shared memory, where a
+// thread finishes one column in plane order.  The operations are
+// reduce_plane's in its order, so the results are the batched kernels' bit
+// for bit.  Outputs go to the mapped scratch a line at a time, then each
+// block stores the call's number in its word there: the host sees the last
+// of them 1.6 us earlier than the stream's completion.
+//
+// A vgh call from Python, before (one-warp blocks, each going through the four
+// planes, and a stream synchronisation) and now, us: 32^3 x 128 FP32 20.8 /
+// 16.3, 64^3 x 1024 23.4 / 18.8, F16 23.8 / 18.4, 48^3 x 512 FP64 44.8 / 23.0;
+// an empty kernel's launch and synchronisation take 8.6 us in C.
+struct PointArgs {
+  const void *coefs;
+  const float *scale;
+  int64_t xs, ys, zs;
+  double start[3], dinv[3], inl[3];
+  float dinvf[3];
+  int lim[3];
+  int ncol, rule, is_complex, out;
+  void *vals, *grads, *hess;
+  unsigned *done, seq;
+};
+
+template <int ST>
+struct PointCfg {
+  static constexpr int VW = ST == ST_F64 ? 1 : CT<ST>::VW, W = 32 * VW;  // columns a thread, a block
+};
+
+template <int ST, bool VGH>
+__global__ void __launch_bounds__(128) k_point(const PointArgs a) {
+  using A = typename CT<ST>::A;
+  constexpr int VW = PointCfg<ST>::VW, W = PointCfg<ST>::W, NY = VGH ? 6 : 1;
+  __shared__ A sw[4][36];
+  __shared__ A sy[4][NY][W];
+  __shared__ A so[VGH ? 13 * W : W];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c0 = blockIdx.x * W;
+  A *w = sw[warp];
+  int idx = 0;
+  if (lane < 3) {
+    A t;
+    cell(a, lane, a.inl[lane], idx, t);
+    bspline_weights<A>(t, w + lane * 12, sizeof(A) == 4 ? (A)a.dinvf[lane] : (A)a.dinv[lane]);
+  }
+  const int ix = __shfl_sync(0xffffffffu, idx, 0), iy = __shfl_sync(0xffffffffu, idx, 1),
+            iz = __shfl_sync(0xffffffffu, idx, 2);
+  __syncwarp();
+  const int col0 = c0 + lane * VW;
+  if (col0 < a.ncol) {
+    constexpr int B = CT<ST>::BYTES;
+    const char *plane = reinterpret_cast<const char *>(a.coefs) + (int64_t)col0 * B +
+                        ((ix + warp) * a.xs + iy * a.ys + iz * a.zs) * B;
+    A c[16][VW];
+#pragma unroll
+    for (int r = 0; r < 16; r++) {
+      const char *row = plane + ((r >> 2) * a.ys + (r & 3) * a.zs) * B;
+      if constexpr (ST == ST_F64) c[r][0] = __ldg(reinterpret_cast<const double *>(row));
+      else load_row<ST>(row, c[r]);
+    }
+    A wz[3][4];
+    z_weights<A>(w, wz);
+#pragma unroll
+    for (int e = 0; e < VW; e++) {
+      A y[6];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const A by = w[12 + j], dby = w[16 + j], d2by = w[20 + j];
+        A z[3];
+#pragma unroll
+        for (int d = 0; d < (VGH ? 3 : 1); d++) {
+          z[d] = c[4 * j][e] * wz[d][0];
+#pragma unroll
+          for (int k = 1; k < 4; k++) z[d] = fmaT(c[4 * j + k][e], wz[d][k], z[d]);
+        }
+        const A yw[6] = {by, dby, d2by, by, dby, by};
+        constexpr int Z[6] = {0, 0, 0, 1, 1, 2};
+#pragma unroll
+        for (int q = 0; q < NY; q++) y[q] = j == 0 ? yw[q] * z[Z[q]] : fmaT(yw[q], z[Z[q]], y[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < NY; q++) sy[warp][q][lane * VW + e] = y[q];
+    }
+  }
+  __syncthreads();
+  const int cn = min(W, a.ncol - c0), c = threadIdx.x;
+  if (c < cn) {
+    constexpr int R[10] = {0, 0, 1, 3, 0, 1, 3, 2, 4, 5};
+    constexpr int X[10] = {0, 1, 0, 0, 2, 1, 1, 0, 0, 0};
+    A o[10];
+#pragma unroll
+    for (int q = 0; q < (VGH ? 10 : 1); q++) {
+      o[q] = w[4 * X[q]] * sy[0][R[q]][c];
+#pragma unroll
+      for (int i = 1; i < 4; i++) o[q] = fmaT(w[4 * X[q] + i], sy[i][R[q]][c], o[q]);
+      if (a.scale) o[q] *= (A)a.scale[c0 + c];
+    }
+    so[c] = o[0];
+    if constexpr (VGH) {
+      // complex columns interleave re/im of one spline in every entry
+      const int n = a.is_complex ? c >> 1 : c, p = a.is_complex ? c & 1 : 0, nc = a.is_complex ? 2 : 1;
+      A *sg = so + W, *sh = so + 4 * W;
+#pragma unroll
+      for (int m = 0; m < 3; m++) sg[nc * (3 * n + m) + p] = o[1 + m];
+      if (a.out == 0) {
+#pragma unroll
+        for (int m = 0; m < 9; m++) sh[nc * (9 * n + m) + p] = o[4 + h9to6(m)];
+      } else if (a.out == 2) {
+        sh[c] = (o[4] + o[7]) + o[9];
+      }
+    }
+  }
+  __syncthreads();
+  auto copy = [&](void *dst, const A *src, int m) {
+    A *d = reinterpret_cast<A *>(dst) + (int64_t)m * c0;
+    for (int i = threadIdx.x; i < m * cn; i += 128) d[i] = src[i];
+  };
+  copy(a.vals, so, 1);
+  if constexpr (VGH) {
+    copy(a.grads, so + W, 3);
+    if (a.out != 3) copy(a.hess, so + 4 * W, a.out == 0 ? 9 : 1);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence_system();  // the block's outputs (ordered before by the barrier) first
+    *(volatile unsigned *)(a.done + blockIdx.x) = a.seq;
+  }
+}
+
+// Scratch of the single-point entries in pinned host memory mapped into the
+// device's address space: a call needs no device-to-host copy.
+static size_t pt_out_bytes(const Table *t) { return 40 * pt_cols(t->ncol) * acc_bytes(t); }
 int point_scratch(Table *t, const char *fn) {
   if (t->pt_host) return 0;
-  const size_t sz = 40 * (size_t)t->ncol * acc_bytes(t);
+  const size_t words = ((size_t)t->ncol + 31) / 32;  // at most one block per 32 columns
+  const size_t sz = pt_out_bytes(t) + words * sizeof(unsigned);
   void *h = nullptr, *d = nullptr;
   if (cudaHostAlloc(&h, sz, cudaHostAllocMapped) != cudaSuccess || cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess) {
     cudaGetLastError();
     if (h) cudaFreeHost(h);
     return fail(EINSPLINE_GB300_ENOMEM, "%s: scratch allocation failed", fn);
   }
+  memset((char *)h + pt_out_bytes(t), 0, words * sizeof(unsigned));
   t->pt_host = h;
   t->pt_dev = d;
+  t->pt_seq = 0;
   return 0;
 }
 
-// Launch shape of a single-point evaluation: one warp per block and as many
-// blocks as the columns need, so a wide table's point is spread over many
-// SMs; the stencil rows of the point are first asked of L2 with bulk
-// prefetches (load mode 1), all 64 at once, unless the table forces a mode.
-int launch_point(Table *t, EvalArgs &a, bool vgh) {
-  const int mode = t->tile_mode >= 0 ? t->tile_mode : 1;
-  return launch_eval(t, a, vgh, t->stream, 32, 1, 1, mode);
+// Waits until every block of call t->pt_seq has stored its number.  A launch
+// that fails never does: after 2 ms the stream's own status decides.
+static int wait_point(Table *t, int blocks, const char *fn) {
+  volatile unsigned *done = (volatile unsigned *)((char *)t->pt_host + pt_out_bytes(t));
+  const auto t0 = std::chrono::steady_clock::now();
+  for (int b = 0; b < blocks; b++)
+    for (unsigned n = 1; done[b] != t->pt_seq; n++)
+      if ((n & 1023) == 0 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(2)) {
+        const cudaError_t e = cudaStreamSynchronize(t->stream);
+        if (e != cudaSuccess) return cuda_check(e, fn);
+        if (done[b] != t->pt_seq) return fail(EINSPLINE_GB300_ECUDA, "%s: the evaluation kernel did not finish", fn);
+      }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return 0;
+}
+
+template <int ST>
+static void launch_point_k(const PointArgs &p, bool vgh, int blocks, cudaStream_t s) {
+  if (vgh) k_point<ST, true><<<blocks, 128, 0, s>>>(p);
+  else k_point<ST, false><<<blocks, 128, 0, s>>>(p);
+}
+
+// One point with outputs in the scratch (a: geometry, position, rule, out and
+// output addresses set), finished on return.  A forced load mode, and
+// double-float arithmetic, take the batched kernels: one warp a block, and
+// (mode 1) L2 asked for all 64 stencil rows before the loads.
+int eval_point_now(Table *t, EvalArgs &a, bool vgh, const char *fn) {
+  if (t->tile_mode >= 0 || kernel_storage(t) == ST_DF) {
+    const int mode = t->tile_mode >= 0 ? t->tile_mode : 1;
+    if (int r = launch_eval(t, a, vgh, t->stream, 32, 1, 1, mode)) return r;
+    if (cudaError_t e = cudaStreamSynchronize(t->stream)) return cuda_check(e, fn);
+    return wait_status(t, fn);
+  }
+  PointArgs p;
+  p.coefs = a.coefs; p.scale = a.scale;
+  p.xs = a.xs; p.ys = a.ys; p.zs = a.zs;
+  for (int i = 0; i < 3; i++) {
+    p.start[i] = a.start[i]; p.dinv[i] = a.dinv[i]; p.inl[i] = a.inl[i];
+    p.dinvf[i] = a.dinvf[i]; p.lim[i] = a.lim[i];
+  }
+  p.ncol = a.ncol; p.rule = a.rule; p.is_complex = a.is_complex; p.out = a.out;
+  p.vals = a.vals; p.grads = a.grads; p.hess = a.hess;
+  if (++t->pt_seq == 0) t->pt_seq = 1;
+  p.done = (unsigned *)((char *)t->pt_dev + pt_out_bytes(t));
+  p.seq = t->pt_seq;
+  const int W = t->storage == ST_F64 ? PointCfg<ST_F64>::W : PointCfg<ST_F32>::W;
+  const int blocks = (a.ncol + W - 1) / W;
+  switch (t->storage) {
+    case ST_F32: launch_point_k<ST_F32>(p, vgh, blocks, t->stream); break;
+    case ST_F16: launch_point_k<ST_F16>(p, vgh, blocks, t->stream); break;
+    case ST_BF16: launch_point_k<ST_BF16>(p, vgh, blocks, t->stream); break;
+    case ST_I16: launch_point_k<ST_I16>(p, vgh, blocks, t->stream); break;
+    default: launch_point_k<ST_F64>(p, vgh, blocks, t->stream); break;
+  }
+  EG_CUDA(cudaGetLastError());
+  count_launch();
+  return wait_point(t, blocks, fn);
 }
 
 }  // namespace eg
@@ -1527,19 +1713,15 @@ void eval_point(S *s, double x, double y, double z, V *vals, V *grads, V *hess, 
   a.out = out;
   a.npts = 1;
   a.vals = t->pt_dev;
-  a.grads = (char *)t->pt_dev + n * rb;
-  a.hess = (char *)t->pt_dev + 4 * n * rb;
-  if (launch_point(t, a, vgh)) return;
-  if (cudaError_t e = cudaStreamSynchronize(t->stream)) {
-    cuda_check(e, fn);
-    return;
-  }
-  if (wait_status(t, fn)) return;
+  const size_t na = pt_cols(t->ncol);
+  a.grads = (char *)t->pt_dev + na * rb;
+  a.hess = (char *)t->pt_dev + 4 * na * rb;
+  if (eval_point_now(t, a, vgh, fn)) return;
   memcpy(vals, t->pt_host, n * rb);
   if (vgh) {
-    memcpy(grads, (char *)t->pt_host + n * rb, 3 * n * rb);
-    if (out == 0) memcpy(hess, (char *)t->pt_host + 4 * n * rb, 9 * n * rb);
-    if (out == 2) memcpy(hess, (char *)t->pt_host + 4 * n * rb, n * rb);
+    memcpy(grads, (char *)t->pt_host + na * rb, 3 * n * rb);
+    if (out == 0) memcpy(hess, (char *)t->pt_host + 4 * na * rb, 9 * n * rb);
+    if (out == 2) memcpy(hess, (char *)t->pt_host + 4 * na * rb, n * rb);
   }
 }
 

@@ -166,7 +166,9 @@ __device__ __forceinline__ void bspline_weights(A t, A *w, A d) {
 //  rule 1 (GPU entries, src/multi_bspline_cuda_s_impl.h:370-384):
 //    u = r * delta_inv (no start offset), i = clamp(floor(u), 0, dim-1),
 //    t = u - floor(u).
-__device__ __forceinline__ void cell(const EvalArgs &a, int ax, double xd, int &idx, float &t) {
+// (Args: EvalArgs, or another struct with its geometry fields.)
+template <typename Args>
+__device__ __forceinline__ void cell(const Args &a, int ax, double xd, int &idx, float &t) {
   const int lim = a.lim[ax];
   if (a.rule == 0) {
     const float u = __double2float_rn(__dmul_rn(__dsub_rn(xd, a.start[ax]), a.dinv[ax]));
@@ -184,7 +186,8 @@ __device__ __forceinline__ void cell(const EvalArgs &a, int ax, double xd, int &
     idx = i; t = __fsub_rn(s, sf);
   }
 }
-__device__ __forceinline__ void cell(const EvalArgs &a, int ax, double xd, int &idx, double &t) {
+template <typename Args>
+__device__ __forceinline__ void cell(const Args &a, int ax, double xd, int &idx, double &t) {
   const int lim = a.lim[ax];
   if (a.rule == 0) {
     const double u = __dmul_rn(__dsub_rn(xd, a.start[ax]), a.dinv[ax]);
