@@ -48,21 +48,21 @@ __global__ void k_iota(int *p, int64_t n) {
   if (i < n) p[i] = (int)i;
 }
 
-// Batches of up to kSmallSort points are ordered by a counting sort on the
-// Morton key of coarse cells (the cell index shifted right by `shift`, at
-// most 16 per axis, 4096 keys), in two launches of S blocks (16, or one per
-// kSortSlice points beyond that), block b owning the b-th slice of the
-// points.  k_sort_keys keys its slice and writes the slice's key counts
+// Points are ordered by a counting sort on the Morton key of coarse cells
+// (the cell index shifted right by `shift`, at most 16 per axis, 4096 keys),
+// in two launches of S blocks (16 to 128, one per kSortSlice points between),
+// block b owning the b-th slice of the points.  k_sort_keys keys its slice and writes the slice's key counts
 // (row b of `hist`); k_sort_scatter gives key k of slice b the offset
 // (points with smaller keys) + (points with key k in earlier slices) and
 // places the slice's points with shared-memory atomics.
 // Points of one key within a slice come out in the order the atomics place
 // them; each point still writes its own output slot, so the results do not
 // depend on that order.  (One block doing all of it was latency-bound at
-// ~28 us for 17k points, an 8-block cluster no faster; the radix sort below,
-// for larger batches, takes three launches, ~40 us at 17k points.)
-constexpr int kSortSlice = 2048;  // most points a slice holds
-constexpr int kSortMinBlocks = 16;
+// ~28 us for 17k points, an 8-block cluster no faster; the radix sort below
+// takes three launches, ~40 us at 17k points and 75 us at 160k, where this
+// takes 25 us: F16 96^3 x 1024 x 160,000 points 2137 -> 2087 us in all.)
+constexpr int kSortSlice = 4096;
+constexpr int kSortMinBlocks = 16, kSortMaxBlocks = 128;
 constexpr int kSortThreads = 1024;
 constexpr int kCoarseKeys = 4096;
 constexpr int kKeysPerThread = kCoarseKeys / kSortThreads;
@@ -170,10 +170,19 @@ static int coarse_shift(const EvalArgs &a) {
   return std::max(0, bits - 4);
 }
 
-static int sort_slices(int64_t n) { return (int)std::max<int64_t>(kSortMinBlocks, (n + kSortSlice - 1) / kSortSlice); }
+static int sort_slices(int64_t n) {
+  return (int)std::min<int64_t>(kSortMaxBlocks, std::max<int64_t>(kSortMinBlocks, (n + kSortSlice - 1) / kSortSlice));
+}
 
-// Scratch of the counting sort of n <= kSmallSort points: perm, the keys,
-// then the slices' key counts.
+// Whether a batch takes the radix sort on whole cells instead: values of FP32
+// tables, whose direct loads gain more from exact neighbours in L1 than the
+// sort costs once there are many points (64^3 x 512, 400,000 points: 1765
+// against 1899 us; vgh, 16-bit and FP64 tables are 1-7 % faster with the
+// counting sort, or equal).
+bool sorts_by_radix(const Table *t, bool vgh, int64_t n) { return n > kSmallSort && !vgh && t->storage == ST_F32; }
+
+// Scratch of the counting sort of n points: perm, the keys, then the slices'
+// key counts.
 size_t small_sort_bytes(int64_t n) {
   return align_up_sz(n * 4, 256) + align_up_sz(n * 2, 256) + (size_t)sort_slices(n) * kCoarseKeys * 4;
 }
@@ -203,7 +212,7 @@ int load_sort_kernels() {
   return 0;
 }
 
-int sort_points(Table *t, const EvalArgs &a, int **perm_out, cudaStream_t s) {
+int sort_points(Table *t, const EvalArgs &a, bool vgh, int **perm_out, cudaStream_t s) {
   const int64_t n = a.npts;
   if (n > INT_MAX) return fail(EINSPLINE_GB300_ESIZE, "sorted evaluation takes at most %d points", INT_MAX);
   int bits = 0;
@@ -212,7 +221,7 @@ int sort_points(Table *t, const EvalArgs &a, int **perm_out, cudaStream_t s) {
     while ((1 << b) <= a.lim[ax]) b++;
     bits = std::max(bits, b);
   }
-  if (n <= kSmallSort) {
+  if (!sorts_by_radix(t, vgh, n)) {
     const size_t need = small_sort_bytes(n);
     if (t->sort_bytes < need) {
       cudaFree(t->sort_dev);
@@ -418,7 +427,7 @@ static int eval_device(Table *t, const einspline_gb300_eval_opts *o, int64_t npt
   a.vals = v; a.grads = g; a.hess = h;
   if (!o->sort || npts <= 1) return launch_eval_ordered(t, a, o->vgh != 0, s);
   int *perm = nullptr;
-  if (int r = sort_points(t, a, &perm, s)) return r;
+  if (int r = sort_points(t, a, o->vgh != 0, &perm, s)) return r;
   a.perm = perm;
   int tx, ty, pb;
   pick_tile(t, o->vgh != 0, npts, tx, ty, pb, true);
@@ -824,7 +833,7 @@ int einspline_gb300_autotune_sorted(einspline_gb300_table *t, int64_t npts, int 
   uniform_points(t, all, npts);
   EvalArgs s = tuning_args(t, all, npts, buf);
   int *perm = nullptr;
-  int r = sort_points(t, s, &perm, t->stream);
+  int r = sort_points(t, s, vgh != 0, &perm, t->stream);
   if (!r) {
     k_gather_pos<<<(unsigned)((W + 255) / 256), 256, 0, t->stream>>>(all, perm, W, win);
     count_launch();

@@ -300,11 +300,12 @@ void order_scratch_init(Table *t);
 void order_scratch_free(Table *t);
 
 // sorting
-int sort_points(Table *t, const EvalArgs &a, int **perm_out, cudaStream_t s);
-// The counting sort of batches of up to kSmallSort points into caller-given
-// scratch of small_sort_bytes(npts) bytes (16-byte aligned; nothing in it
-// has to start at zero).
+int sort_points(Table *t, const EvalArgs &a, bool vgh, int **perm_out, cudaStream_t s);
+// The counting sort of up to INT_MAX points into caller-given scratch of
+// small_sort_bytes(npts) bytes (16-byte aligned; nothing in it has to start
+// at zero).  Up to kSmallSort points everything is sorted that way.
 constexpr int64_t kSmallSort = 131072;
+bool sorts_by_radix(const Table *t, bool vgh, int64_t n);
 size_t small_sort_bytes(int64_t n);
 int small_sort_into(const EvalArgs &a, void *scratch, int **perm_out, cudaStream_t s);
 // Morton key of each point's cell and its index (defined in api_ext.cu).

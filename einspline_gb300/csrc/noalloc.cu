@@ -180,9 +180,9 @@ extern "C" int einspline_gb300_eval_3d_sorted_noalloc(einspline_gb300_table *t, 
 
   int tx, ty, pb;
   pick_tile(t, o->vgh != 0, npts, tx, ty, pb, true);
-  // Batches of up to kSmallSort points: the two-launch counting sort, whose
-  // scratch (under 2 MB) is written before it is read.
-  if (npts <= kSmallSort && small_sort_bytes(npts) <= kScratchBytes) {
+  // The two-launch counting sort, whose scratch (under 3 MB) is written before
+  // it is read; large batches of FP32 values take the radix sort.
+  if (!sorts_by_radix(t, o->vgh != 0, npts) && small_sort_bytes(npts) <= kScratchBytes) {
     int *perm = nullptr;
     if (int r = small_sort_into(a, scratch, &perm, s)) return r;
     a.perm = perm;

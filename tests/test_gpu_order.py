@@ -171,3 +171,31 @@ def test_fp64_tables_keep_their_order():
                 if b is not None:
                     assert torch.equal(a[p0:p0 + 3 * SMALL], b)
     _tables.clear()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,storage,vgh", [("s", api.STORE_NATIVE, False), ("s", api.STORE_F16, True),
+                                              ("s", api.STORE_NATIVE, True), ("d", api.STORE_NATIVE, False)])
+@pytest.mark.parametrize("n", [131072, 131073, 262144])
+def test_large_sorted_batches(kind, storage, vgh, n):
+    """Around the size where values of FP32 tables turn to the radix sort and
+    everything else goes on with the counting sort: both sorted entries give
+    the unsorted bits."""
+    torch = pytest.importorskip("torch")
+    G = api.MultiUBspline3D(kind, [(0.0, 1.0, 33), (0.0, 1.0, 9), (0.0, 1.0, 20)], PER, 6, storage=storage)
+    dt = torch.float32 if kind == "s" else torch.float64
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    G.set_device(0, torch.rand((6,) + G.M, generator=g, device="cuda", dtype=dt) - 0.5)
+    pos = points(torch, n, torch.float64)
+    ref = G.eval(pos, vgh=vgh)
+    got = G.eval(pos, vgh=vgh, sort=True)
+    out = [torch.full_like(x, 3.0) if x is not None else None for x in ref]
+    o = G.opts(vgh, True, 0, 0, True)
+    p = lambda t: C.c_void_p(t.data_ptr() if t is not None else 0)  # noqa: E731
+    L.load().einspline_gb300_eval_3d_sorted_noalloc(G.table, C.byref(o), n, p(pos), p(out[0]), p(out[1]), p(out[2]),
+                                                    C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    L.check()
+    for a, b, c in zip(ref, got, out):
+        if a is not None:
+            assert torch.equal(a, b) and torch.equal(a, c)
