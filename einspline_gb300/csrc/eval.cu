@@ -284,6 +284,38 @@ __global__ void __launch_bounds__(256) k_eval(const EvalArgs a) {
   }
 }
 
+// The points and columns a thread of the wide value kernel goes through.  A
+// full tile has a thread for each VW columns of a point.  The last tile of a
+// table whose columns do not fill it (777 columns in tiles of 256 leave 9) has
+// fewer columns than threads: there the (point, columns) pairs of the block's
+// points are dealt to all threads in turn.  I16 56 x 60 x 52 x 777, 24,000
+// points: 264 -> 235 us (7 of these by decode2).  The other pipelined kernels
+// do not deal: their tiles are narrower, or in vgh a block-wide point index is
+// worth the 2-5 % that a thread's own costs.
+struct ColumnWalk {
+  int point, lane, lanes, dp, dl;
+  __device__ __forceinline__ ColumnWalk(int cols, int nthr, int vw) {
+    lanes = min(nthr, (cols + vw - 1) / vw);
+    point = threadIdx.x / lanes;
+    lane = threadIdx.x - point * lanes;
+    dp = nthr / lanes;
+    dl = nthr - dp * lanes;
+  }
+  __device__ __forceinline__ void next() {
+    point += dp;
+    lane += dl;
+    if (lane >= lanes) {
+      lane -= lanes;
+      point++;
+    }
+  }
+  // (point, columns) pairs this thread, at its first, has of pn points'
+  __device__ __forceinline__ int count(int pn) const {
+    const int n = pn * lanes - (point * lanes + lane), step = dp * lanes + dl;
+    return n > 0 ? (n + step - 1) / step : 0;
+  }
+};
+
 // Pipelined variant: a stage is one x-plane (16 stencil rows) of one point.
 // Each thread copies its own columns of the rows of stage s+2 into shared
 // memory with asynchronous copies while it reduces stage s, so the bytes in
@@ -314,19 +346,26 @@ __device__ __forceinline__ void eval_pipe_body(const EvalArgs &a) {
       reinterpret_cast<const int64_t *>(smem + smem_w_bytes(a.pb, sizeof(A)) + align_up((size_t)a.pb * 12, 8));
   unsigned char *pipe = smem + align_up(smem_total(a.pb, sizeof(A)), 16);
 
-  const int col0 = (tile * blockDim.x + threadIdx.x) * VW;
-  if (col0 >= a.ncol) return;
-  const char *cbase = reinterpret_cast<const char *>(a.coefs) + (int64_t)col0 * CT<ST>::BYTES;
+  constexpr bool DEAL = WIDE && !VGH;
+  int col0 = (tile * blockDim.x + threadIdx.x) * VW, S = pn * 4;
+  const int c_first = tile * nthr * VW;
+  // dealt: the pair this thread copies and, behind it, the one it reduces
+  ColumnWalk in(DEAL ? a.ncol - c_first : 1, nthr, VW), it = in;
+  if constexpr (DEAL) S = in.count(pn) * 4;
+  else if (col0 >= a.ncol) return;
+  const char *cbase = reinterpret_cast<const char *>(a.coefs) + (int64_t)(DEAL ? c_first : col0) * CT<ST>::BYTES;
   const int64_t xsb = a.xs * CT<ST>::BYTES, ysb = a.ys * CT<ST>::BYTES, zsb = a.zs * CT<ST>::BYTES;
   const unsigned my = (unsigned)__cvta_generic_to_shared(pipe + (size_t)threadIdx.x * RB);
   const unsigned row_step = (unsigned)(nthr * RB), slot_step = 16u * row_step;
-  const int S = pn * 4;
   auto issue = [&](int st) {
-    const int pp = st >> 2, i = st & 3;
+    const int pp = DEAL ? in.point : st >> 2, i = st & 3;
     const char *plane = cbase + (sidx[3 * pp] + i) * xsb + sidx[3 * pp + 1] * ysb + sidx[3 * pp + 2] * zsb;
+    if constexpr (DEAL) plane += in.lane * VW * CT<ST>::BYTES;
     const unsigned dst = my + (unsigned)(st % NS) * slot_step;
 #pragma unroll
     for (int r = 0; r < 16; r++) cp_async<RB>(dst + r * row_step, plane + (r >> 2) * ysb + (r & 3) * zsb);
+    if constexpr (DEAL)
+      if (i == 3) in.next();
   };
 #pragma unroll
   for (int st = 0; st < NS - 1; st++) {
@@ -339,7 +378,7 @@ __device__ __forceinline__ void eval_pipe_body(const EvalArgs &a) {
     if (st + NS - 1 < S) issue(st + NS - 1);
     cp_async_commit();
     cp_async_wait<NS - 1>();
-    const int pp = st >> 2, i = st & 3;
+    const int pp = DEAL ? it.point : st >> 2, i = st & 3;
     const A *w = sw + pp * 36;
     if (i == 0) z_weights<A>(w, wz);
     const unsigned char *slot = pipe + (size_t)(st % NS) * slot_step + (size_t)threadIdx.x * RB;
@@ -349,8 +388,13 @@ __device__ __forceinline__ void eval_pipe_body(const EvalArgs &a) {
           const Raw *rp = reinterpret_cast<const Raw *>(slot + (j * 4 + k) * row_step);
           if (WIDE) {
             A lo[CT<ST>::VW], hi[CT<ST>::VW];
-            CT<ST>::decode(rp[0], lo);
-            CT<ST>::decode(rp[1], hi);
+            if constexpr (ST == ST_I16 && !VGH) {
+              CT<ST>::decode2(rp[0], lo);
+              CT<ST>::decode2(rp[1], hi);
+            } else {
+              CT<ST>::decode(rp[0], lo);
+              CT<ST>::decode(rp[1], hi);
+            }
 #pragma unroll
             for (int e = 0; e < CT<ST>::VW; e++) { c[e] = lo[e]; c[CT<ST>::VW + e] = hi[e]; }
           } else {
@@ -359,6 +403,10 @@ __device__ __forceinline__ void eval_pipe_body(const EvalArgs &a) {
         },
         o);
     if (i == 3) {
+      if constexpr (DEAL) {
+        col0 = c_first + it.lane * VW;
+        it.next();
+      }
       if constexpr (ST == ST_DF) {
         double od[10][VW];
 #pragma unroll
@@ -1223,6 +1271,11 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   // waves on, 4 points a lane are up to 10 % faster), for FP64, which its
   // arithmetic bounds, below one.
   if (b.mode == 0 && (!vgh || t->storage == ST_F64) && (a.npts + pb - 1) / pb * b.ntiles < (t->storage == ST_F64 ? 1 : 4) * wave) pb = (int)block.y;
+  // groups' blocks; the wide value kernel deals the columns of a ragged last
+  // tile to all its threads, so that tile counts by its share of the columns
+  const bool dealt = b.mode == 3 && !vgh;
+  const int64_t tcols = (int64_t)tx * elems_per_thread(t) * 2;
+  auto blocks_of = [&](int64_t groups) { return dealt ? (groups * a.ncol + tcols - 1) / tcols : groups * b.ntiles; };
   const int64_t full = (a.npts + pb - 1) / pb * b.ntiles;
   if (full >= wave) {
     // between one and two waves of the copy pipelines' blocks: the size whose
@@ -1231,7 +1284,7 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
     if (b.mode < 2 || b.mode > 4 || full > 2 * wave) return;
     int64_t best = INT64_MAX;
     for (int p = pb, p0 = pb; p >= (p0 + 1) / 2; p--) {
-      const int64_t cost = ((a.npts + p - 1) / p * b.ntiles + wave - 1) / wave * p;
+      const int64_t cost = (blocks_of((a.npts + p - 1) / p) + wave - 1) / wave * p;
       if (cost < best) {
         best = cost;
         pb = p;

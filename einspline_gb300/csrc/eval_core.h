@@ -53,6 +53,43 @@ __device__ __forceinline__ dfl to_dfl(double x) {
 }
 __device__ __forceinline__ double to_double(dfl x) { return __dadd_rn((double)x.h, (double)x.l); }
 
+// ------------------------------------------------------------ packed FP32
+// Blackwell's 2-wide FP32 instructions (PTX fma.rn.f32x2 and its like):
+// each lane is the IEEE round-to-nearest operation of the scalar code, so a
+// pair of columns sharing one weight costs one instruction instead of two
+// and gives bit-identical results.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void upk2(f32x2 r, float &a, float &b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 neg2(f32x2 a) { return a ^ 0x8000000080000000ull; }
+
 // ------------------------------------------------------------ coefficient types
 // Raw is what one thread reads per stencil row (VW stored reals); decode
 // turns it into VW accumulator values.
@@ -90,12 +127,23 @@ template <> struct CT<ST_I16> {
   static constexpr int VW = 4, BYTES = 2;
   // A biased 16-bit pattern u placed under the exponent of 2^23 is the float
   // 2^23 + u; subtracting 2^23 + bias is exact and leaves the integer.
+  __device__ static __forceinline__ float at(unsigned u, unsigned sel) {
+    return __uint_as_float(__byte_perm(u, 0x4B000000u, sel));
+  }
+  static constexpr float kOff = 8388608.0f + (float)kI16Bias;
   __device__ static __forceinline__ void decode(const Raw &x, float (&v)[4]) {
-    const float off = 8388608.0f + (float)kI16Bias;
-    v[0] = __int_as_float(__byte_perm(x.x, 0x4B000000u, 0x7610)) - off;
-    v[1] = __int_as_float(__byte_perm(x.x, 0x4B000000u, 0x7632)) - off;
-    v[2] = __int_as_float(__byte_perm(x.y, 0x4B000000u, 0x7610)) - off;
-    v[3] = __int_as_float(__byte_perm(x.y, 0x4B000000u, 0x7632)) - off;
+    v[0] = at(x.x, 0x7610) - kOff;
+    v[1] = at(x.x, 0x7632) - kOff;
+    v[2] = at(x.y, 0x7610) - kOff;
+    v[3] = at(x.y, 0x7632) - kOff;
+  }
+  // The same, two columns a subtraction: 3 % of the wide value kernel (64^3 x
+  // 1024, 24,000 sorted points: 250 -> 242 us); in the vgh kernels, where
+  // registers are short, the pairs cost 1.5 %.
+  __device__ static __forceinline__ void decode2(const Raw &x, float (&v)[4]) {
+    const f32x2 off = pk2(kOff, kOff);
+    upk2(sub2(pk2(at(x.x, 0x7610), at(x.x, 0x7632)), off), v[0], v[1]);
+    upk2(sub2(pk2(at(x.y, 0x7610), at(x.y, 0x7632)), off), v[2], v[3]);
   }
 };
 template <> struct CT<ST_F64> {
@@ -206,43 +254,7 @@ __device__ __forceinline__ void cell(const Args &a, int ax, double xd, int &idx,
   }
 }
 
-// ------------------------------------------------------------ packed FP32
-// Blackwell's 2-wide FP32 instructions (PTX fma.rn.f32x2 / mul.rn.f32x2):
-// each lane is the IEEE round-to-nearest operation of the scalar code, so a
-// pair of columns sharing one weight costs one instruction instead of two
-// and gives bit-identical results.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pk2(float a, float b) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void upk2(f32x2 r, float &a, float &b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r));
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ f32x2 neg2(f32x2 a) { return a ^ 0x8000000080000000ull; }
-
+// ------------------------------------------------------------ packed double-float
 // Two double-float values (one per column) in packed form: the same
 // operations as dfl's, lane by lane.
 struct dfl2 {
