@@ -1161,11 +1161,13 @@ static int shape_kernel(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb,
     *smem = tc_smem(pb);
   } else if (a.mode == 4) {
     ty = 1;
+    const int es = is16(t->storage) ? 2 : (ks == ST_F32 ? 4 : 8);
+    // whole boxes, which hold at most 256 columns
+    if (tx > 16 * es) tx = tx / (16 * es) * (16 * es);
     // narrower tiles where the stage buffers would not fit in shared memory
     const int stages = ks == ST_DF ? TmaStages<ST_DF>::value : kTmaStages;
     while (tx > 32 && tma_smem(pb, acc_bytes(t), tx, stages) > max_smem_optin()) tx /= 2;
     a.ntiles = (a.ncol + tx * VW - 1) / (tx * VW);
-    const int es = is16(t->storage) ? 2 : (ks == ST_F32 ? 4 : 8);
     a.box_bytes = tx * 16 < 256 * es ? tx * 16 : 256 * es;
     *smem = tma_smem(pb, acc_bytes(t), tx, stages);
   } else if (a.mode >= 2) {
