@@ -44,12 +44,75 @@ __device__ __forceinline__ void st_vec(double *p, const double (&v)[N]) {
 #pragma unroll
   for (int c = 0; c < N / 2; c++) __stcs(reinterpret_cast<double2 *>(p) + c, make_double2(v[2 * c], v[2 * c + 1]));
 }
+// The lanes of a warp storing runs that follow each other in memory (lane i's
+// columns before lane i + 1's).
+struct LaneRuns {
+  unsigned mask;    // the lanes that store
+  bool first;       // no lane stores what lies before this run
+  bool next_full;   // the next lane stores a whole run
+  // columns col0 .. col0 + vw - 1 of lane threadIdx.x & 31
+  __device__ __forceinline__ LaneRuns(int col0, int vw, int ncol) {
+    const int lane = threadIdx.x & 31, n = min(32, (ncol - (col0 - lane * vw) + vw - 1) / vw);
+    mask = n == 32 ? 0xffffffffu : (1u << n) - 1u;
+    first = lane == 0;
+    next_full = lane + 1 < n && col0 + 2 * vw <= ncol;
+  }
+};
+// A run whose address lies 4 * LEAD bytes before a 16-byte boundary: 16-byte
+// stores from that boundary on, the last of them with the next lane's first
+// LEAD elements (h), which that lane leaves out.
+template <int LEAD, int N>
+__device__ __forceinline__ void st_shifted(float *p, const float (&v)[N], const float (&h)[3], const LaneRuns &w) {
+  if (w.first) {
+#pragma unroll
+    for (int e = 0; e < LEAD; e++) p[e] = v[e];
+  }
+#pragma unroll
+  for (int c = 0; c + 1 < N / 4; c++)
+    __stcs(reinterpret_cast<float4 *>(p + LEAD) + c,
+           make_float4(v[LEAD + 4 * c], v[LEAD + 4 * c + 1], v[LEAD + 4 * c + 2], v[LEAD + 4 * c + 3]));
+  if (w.next_full) {
+    float t[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) t[e] = e < 4 - LEAD ? v[N - 4 + LEAD + (e < 4 - LEAD ? e : 0)] : h[e < 4 - LEAD ? 0 : e - 4 + LEAD];
+    __stcs(reinterpret_cast<float4 *>(p + LEAD + N - 4), make_float4(t[0], t[1], t[2], t[3]));
+  } else {
+#pragma unroll
+    for (int e = LEAD + N - 4; e < N; e++) p[e] = v[e];
+  }
+}
+// One lane's run of N reals at p (N a multiple of 4, the same offset from a
+// 16-byte boundary on every lane): 16-byte stores at every offset.  An odd
+// number of splines puts three points in four off the boundary, where each
+// real was a store of its own and a warp's store touched 32 sectors; one() is
+// that store, still taken by the lane at the table's ragged end.
+// 24,000 points, vgh: I16 48^3 x 777: 735 -> 529 us; FP32 45^3 x 203: 168 ->
+// 156, in the CPU layout 242 -> 169.
+template <int N, typename One>
+__device__ __forceinline__ void st_run(float *p, const float (&v)[N], bool full, const LaneRuns &w, One one) {
+  const unsigned off = (unsigned)reinterpret_cast<uintptr_t>(p) & 15u;
+  if (full && off == 0) {
+    st_vec<N>(p, v);
+    return;
+  }
+  float h[3] = {};
+  if (off != 0) {
+#pragma unroll
+    for (int e = 0; e < 3; e++) h[e] = __shfl_down_sync(w.mask, v[e], 1);
+  }
+  if (!full) one();
+  else if (off == 12) st_shifted<1>(p, v, h, w);
+  else if (off == 8) st_shifted<2>(p, v, h, w);
+  else st_shifted<3>(p, v, h, w);
+}
 // Index of Hessian entry m (row-major 3x3) among (xx, xy, xz, yy, yz, zz).
 __device__ __forceinline__ int h9to6(int m) {
   return (m == 0) ? 0 : (m == 1 || m == 3) ? 1 : (m == 2 || m == 6) ? 2 : (m == 4) ? 3 : (m == 5 || m == 7) ? 4 : 5;
 }
 
-template <typename A, int VW, bool VGH, bool SCALE = true>
+// SHIFT: rows may start off a 16-byte boundary, and the warp's lanes are here
+// together for one point.
+template <typename A, int VW, bool VGH, bool SCALE = true, bool SHIFT = false>
 __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col0, A (&o)[10][VW]) {
   if (SCALE && a.scale) {
     float sc[VW];
@@ -86,15 +149,24 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
   A *vp = a.vals_pp ? (A *)a.vals_pp[src] : (A *)a.vals + src * a.vstride;
   // vector stores need whole 16-byte groups of columns in this thread
   const bool full = (sizeof(A) == 8 ? VW % 2 == 0 : VW % 4 == 0) && col0 + VW <= a.ncol;
+  const LaneRuns w(col0, VW, a.ncol);
+  auto put = [&](A *p, const auto &v, auto one) {
+    if constexpr (SHIFT && VW % 4 == 0) {
+      st_run(p, v, full, w, one);
+    } else {
+      if (full && al16(p)) st_vec(p, v);
+      else one();
+    }
+  };
   {
     A v[VW];
 #pragma unroll
     for (int e = 0; e < VW; e++) v[e] = o[0][e];
-    if (full && al16(vp + col0)) st_vec<VW>(vp + col0, v);
-    else
+    put(vp + col0, v, [&] {
 #pragma unroll
       for (int e = 0; e < VW; e++)
         if (col0 + e < a.ncol) vp[col0 + e] = v[e];
+    });
   }
   if (!VGH) return;
   if (a.out == 1) {
@@ -123,11 +195,11 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
 #pragma unroll
     for (int r = 0; r < 4; r++) {
       A *rp = gl + r * a.lrow + col0;
-      if (full && al16(rp)) st_vec<VW>(rp, row[r]);
-      else
+      put(rp, row[r], [&] {
 #pragma unroll
         for (int e = 0; e < VW; e++)
           if (col0 + e < a.ncol) rp[e] = row[r][e];
+      });
     }
     return;
   }
@@ -147,8 +219,7 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
         g[idx] = o[1 + c][e];
       }
     A *gb = gp + 3 * (int64_t)col0;
-    if (full && al16(gb)) st_vec<3 * VW>(gb, g);
-    else
+    put(gb, g, [&] {
 #pragma unroll
       for (int e = 0; e < VW; e++)
         if (col0 + e < a.ncol)
@@ -157,6 +228,7 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
             const int idx = cpx_cpu ? 6 * (e >> 1) + 2 * c + (e & 1) : 3 * e + c;
             gb[idx] = g[idx];
           }
+    });
   }
   if (a.out == 3) return;
   if (a.out == 2) {
@@ -165,11 +237,11 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
 #pragma unroll
     for (int e = 0; e < VW; e++) l[e] = (o[4][e] + o[7][e]) + o[9][e];
     A *lb = hp + col0;
-    if (full && al16(lb)) st_vec<VW>(lb, l);
-    else
+    put(lb, l, [&] {
 #pragma unroll
       for (int e = 0; e < VW; e++)
         if (col0 + e < a.ncol) lb[e] = l[e];
+    });
     return;
   }
   if (a.layout == 0) {
@@ -179,13 +251,13 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
 #pragma unroll
       for (int q = 0; q < 6; q++) h[6 * e + q] = o[4 + q][e];
     A *hb = hp + 6 * (int64_t)col0;
-    if (full && al16(hb)) st_vec<6 * VW>(hb, h);
-    else
+    put(hb, h, [&] {
 #pragma unroll
       for (int e = 0; e < VW; e++)
         if (col0 + e < a.ncol)
 #pragma unroll
           for (int q = 0; q < 6; q++) hb[6 * e + q] = h[6 * e + q];
+    });
   } else {
     A h[9 * VW];
 #pragma unroll
@@ -196,8 +268,7 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
         h[idx] = o[4 + h9to6(m)][e];
       }
     A *hb = hp + 9 * (int64_t)col0;
-    if (full && al16(hb)) st_vec<9 * VW>(hb, h);
-    else
+    put(hb, h, [&] {
 #pragma unroll
       for (int e = 0; e < VW; e++)
         if (col0 + e < a.ncol)
@@ -206,10 +277,11 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
             const int idx = cpx ? 18 * (e >> 1) + 2 * m + (e & 1) : 9 * e + m;
             hb[idx] = h[idx];
           }
+    });
   }
 }
 
-template <int ST, bool VGH>
+template <int ST, bool VGH, bool SHIFT>
 __global__ void __launch_bounds__(256) k_eval(const EvalArgs a) {
   using A = typename CT<ST>::A;
   constexpr int VW = CT<ST>::VW;
@@ -282,7 +354,7 @@ __global__ void __launch_bounds__(256) k_eval(const EvalArgs a) {
         for (int e = 0; e < VW; e++) od[q][e] = to_double(o[q][e]);
       epilogue<double, VW, VGH>(a, ssrc[pp], col0, od);
     } else {
-      epilogue<A, VW, VGH>(a, ssrc[pp], col0, o);
+      epilogue<A, VW, VGH, true, SHIFT>(a, ssrc[pp], col0, o);
     }
   }
 }
@@ -327,7 +399,7 @@ struct ColumnWalk {
 // needed.  WIDE (16-bit tables): 8 columns and one 16-byte copy per thread
 // and row instead of 4 columns and 8 bytes.  Same arithmetic, same order as
 // k_eval.
-template <int ST, bool VGH, bool WIDE>
+template <int ST, bool VGH, bool WIDE, bool SHIFT>
 __device__ __forceinline__ void eval_pipe_body(const EvalArgs &a) {
   using A = typename CT<ST>::A;
   using Raw = typename CT<ST>::Raw;
@@ -418,15 +490,15 @@ __device__ __forceinline__ void eval_pipe_body(const EvalArgs &a) {
           for (int e = 0; e < VW; e++) od[q][e] = to_double(o[q][e]);
         epilogue<double, VW, VGH>(a, ssrc[pp], col0, od);
       } else {
-        epilogue<A, VW, VGH>(a, ssrc[pp], col0, o);
+        epilogue<A, VW, VGH, true, SHIFT>(a, ssrc[pp], col0, o);
       }
     }
   }
 }
 
-template <int ST, bool VGH, bool WIDE>
+template <int ST, bool VGH, bool WIDE, bool SHIFT>
 __global__ void __launch_bounds__(256) k_eval_pipe(const EvalArgs a) {
-  eval_pipe_body<ST, VGH, WIDE>(a);
+  eval_pipe_body<ST, VGH, WIDE, SHIFT>(a);
 }
 
 // The double-float variant is held to 128 registers (ptxas fits it without
@@ -437,7 +509,7 @@ __global__ void __launch_bounds__(256) k_eval_pipe(const EvalArgs a) {
 // warps, scheduled differently).
 template <bool VGH>
 __global__ void __maxnreg__(128) k_eval_pipe_df(const EvalArgs a) {
-  eval_pipe_body<ST_DF, VGH, false>(a);
+  eval_pipe_body<ST_DF, VGH, false, false>(a);
 }
 
 // Tensor-map pipeline: a stage is again one x-plane of one point, but the
@@ -452,7 +524,7 @@ __global__ void __maxnreg__(128) k_eval_pipe_df(const EvalArgs a) {
 // Same arithmetic, same order as k_eval.  A wait that runs out sets
 // a.wait_err, leaves the loop on every warp, and thread 0 then waits (again
 // bounded) for the copies it issued before the block exits.
-template <int ST, bool VGH>
+template <int ST, bool VGH, bool SHIFT>
 __global__ void __launch_bounds__(256) k_eval_tma(const __grid_constant__ EvalArgs a) {
   using A = typename CT<ST>::A;
   using Raw = typename CT<ST>::Raw;
@@ -557,7 +629,7 @@ __global__ void __launch_bounds__(256) k_eval_tma(const __grid_constant__ EvalAr
             for (int e = 0; e < VW; e++) od[q][e] = to_double(o[q][e]);
           epilogue<double, VW, VGH>(a, ssrc[pp], col0, od);
         } else {
-          epilogue<A, VW, VGH>(a, ssrc[pp], col0, o);
+          epilogue<A, VW, VGH, true, SHIFT>(a, ssrc[pp], col0, o);
         }
       }
     }
@@ -1034,27 +1106,43 @@ void fill_eval_geometry(const Table *t, EvalArgs &a) {
 // 4 shared-memory pipeline fed by tensor-map (TMA) copies.
 // (IEEE FP64 has only the direct-load kernel; the double-float path has the
 // direct, the 4-column pipelined and the TMA kernels.)
-template <int ST, bool VGH>
-static const void *kernel_for(int mode) {
+template <int ST, bool VGH, bool SHIFT>
+static const void *kernel_as(int mode) {
   if constexpr (ST != ST_F64) {
-    if (mode == 4) return (const void *)k_eval_tma<ST, VGH>;
+    if (mode == 4) return (const void *)k_eval_tma<ST, VGH, SHIFT>;
     if constexpr (ST == ST_DF) {
       if (mode == 2 || mode == 3) return (const void *)k_eval_pipe_df<VGH>;
     } else {
       if constexpr (ST == ST_F16 || ST == ST_BF16)
         if (mode == 5) return (const void *)k_eval_tc<ST, VGH>;
-      if (mode == 2) return (const void *)k_eval_pipe<ST, VGH, false>;
-      if (mode == 3) return (const void *)k_eval_pipe<ST, VGH, (ST == ST_F16 || ST == ST_BF16 || ST == ST_I16)>;
+      if (mode == 2) return (const void *)k_eval_pipe<ST, VGH, false, SHIFT>;
+      if (mode == 3) return (const void *)k_eval_pipe<ST, VGH, is16(ST), SHIFT>;
     }
   }
-  return (const void *)k_eval<ST, VGH>;
+  return (const void *)k_eval<ST, VGH, SHIFT>;
 }
-
-template <int ST, bool VGH>
-static cudaError_t launch_k(const EvalArgs &a, unsigned grid, dim3 block, size_t smem, cudaStream_t s) {
-  const void *f = kernel_for<ST, VGH>(a.mode);
-  void *args[] = {const_cast<EvalArgs *>(&a)};
-  return cudaLaunchKernel(f, dim3(grid), block, args, smem, s);
+template <int ST>
+static const void *kernel_for(bool vgh, int mode, bool shift) {
+  if constexpr (ST != ST_F64 && ST != ST_DF)
+    if (vgh && shift) return kernel_as<ST, true, true>(mode);
+  return vgh ? kernel_as<ST, true, false>(mode) : kernel_as<ST, false, false>(mode);
+}
+// Whether a launch takes the vgh kernels' SHIFT variants, which are for rows
+// that may start off a 16-byte boundary.  They are not the only variants: the
+// aligned case loses 1-5 % to them (I16 48^3 x 776: 490 against 510 us;
+// complex FP32 64^3 x 256 sorted 378 against 382).  Rows given one pointer a
+// point are taken to be aligned; either variant stores any row rightly.
+// Direct loads gain from 256 points on (FP32 45^3 x 201: 48 points 4.5
+// against 4.8 us shifted, 1000 points 11.6 against 9.6), and not from rows at
+// odd multiples of 8 bytes in the GPU layout (complex FP32 40^3 x 101: 24,000
+// points 137 against 140; in the CPU layout 198 against 154).
+static bool shifted_rows(const EvalArgs &a) {
+  if (a.vals_pp || a.grads_pp || a.hess_pp) return false;
+  const uintptr_t base = reinterpret_cast<uintptr_t>(a.vals) | reinterpret_cast<uintptr_t>(a.grads) |
+                         reinterpret_cast<uintptr_t>(a.hess);
+  const int64_t strides = a.vstride | a.gstride | a.hstride;
+  if (a.mode == 0 && (a.npts < 256 || (a.layout == 0 && !(base & 7) && !(strides & 1)))) return false;
+  return (base & 15) || (strides & 3);
 }
 
 // The kernel type of a table's launches: its storage, or the double-float
@@ -1176,13 +1264,14 @@ static int shape_kernel(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb,
     *smem = align_up(*smem, 16) + pipe_bytes(tx, rb, pipe_stages(ks, a.mode == 3 && is16(ks)));
   }
   *block = dim3(tx, ty);
+  const bool shift = shifted_rows(a);
   switch (ks) {
-    case ST_DF: *func = vgh ? kernel_for<ST_DF, true>(a.mode) : kernel_for<ST_DF, false>(a.mode); break;
-    case ST_F32: *func = vgh ? kernel_for<ST_F32, true>(a.mode) : kernel_for<ST_F32, false>(a.mode); break;
-    case ST_F16: *func = vgh ? kernel_for<ST_F16, true>(a.mode) : kernel_for<ST_F16, false>(a.mode); break;
-    case ST_BF16: *func = vgh ? kernel_for<ST_BF16, true>(a.mode) : kernel_for<ST_BF16, false>(a.mode); break;
-    case ST_I16: *func = vgh ? kernel_for<ST_I16, true>(a.mode) : kernel_for<ST_I16, false>(a.mode); break;
-    default: *func = vgh ? kernel_for<ST_F64, true>(a.mode) : kernel_for<ST_F64, false>(a.mode); break;
+    case ST_DF: *func = kernel_for<ST_DF>(vgh, a.mode, shift); break;
+    case ST_F32: *func = kernel_for<ST_F32>(vgh, a.mode, shift); break;
+    case ST_F16: *func = kernel_for<ST_F16>(vgh, a.mode, shift); break;
+    case ST_BF16: *func = kernel_for<ST_BF16>(vgh, a.mode, shift); break;
+    case ST_I16: *func = kernel_for<ST_I16>(vgh, a.mode, shift); break;
+    default: *func = kernel_for<ST_F64>(vgh, a.mode, shift); break;
   }
   return 0;
 }
@@ -1355,21 +1444,8 @@ int launch_eval(Table *t, EvalArgs &a, bool vgh, cudaStream_t s, int tx, int ty,
   }
   const int64_t blocks = plan_groups(a, func, block, smem) * a.ntiles;
   if (blocks > INT_MAX) return fail(EINSPLINE_GB300_ESIZE, "too many points in one call (%lld)", (long long)a.npts);
-  cudaError_t e;
-  switch (kernel_storage(t)) {
-    case ST_DF: e = vgh ? launch_k<ST_DF, true>(a, (unsigned)blocks, block, smem, s)
-                        : launch_k<ST_DF, false>(a, (unsigned)blocks, block, smem, s); break;
-    case ST_F32: e = vgh ? launch_k<ST_F32, true>(a, (unsigned)blocks, block, smem, s)
-                         : launch_k<ST_F32, false>(a, (unsigned)blocks, block, smem, s); break;
-    case ST_F16: e = vgh ? launch_k<ST_F16, true>(a, (unsigned)blocks, block, smem, s)
-                         : launch_k<ST_F16, false>(a, (unsigned)blocks, block, smem, s); break;
-    case ST_BF16: e = vgh ? launch_k<ST_BF16, true>(a, (unsigned)blocks, block, smem, s)
-                          : launch_k<ST_BF16, false>(a, (unsigned)blocks, block, smem, s); break;
-    case ST_I16: e = vgh ? launch_k<ST_I16, true>(a, (unsigned)blocks, block, smem, s)
-                         : launch_k<ST_I16, false>(a, (unsigned)blocks, block, smem, s); break;
-    default: e = vgh ? launch_k<ST_F64, true>(a, (unsigned)blocks, block, smem, s)
-                     : launch_k<ST_F64, false>(a, (unsigned)blocks, block, smem, s); break;
-  }
+  void *args[] = {&a};
+  const cudaError_t e = cudaLaunchKernel(func, dim3((unsigned)blocks), block, args, smem, s);
   count_launch();
   if (e != cudaSuccess) return cuda_check(e, "evaluation kernel launch");
   return 0;
@@ -1386,12 +1462,15 @@ int load_eval_kernel(Table *t, bool vgh, bool sorted) {
     int tx, ty, pb;
     a.npts = n;
     pick_tile(t, vgh, n, tx, ty, pb, sorted);
-    const void *func;
-    dim3 block;
-    size_t smem;
-    if (int r = shape_launch(t, a, vgh, tx, ty, pb, &func, &block, &smem)) return r;
-    cudaFuncAttributes fa;
-    EG_CUDA(cudaFuncGetAttributes(&fa, func));
+    // and on where the output rows start
+    for (a.vstride = 0; a.vstride < 2; a.vstride++) {
+      const void *func;
+      dim3 block;
+      size_t smem;
+      if (int r = shape_launch(t, a, vgh, tx, ty, pb, &func, &block, &smem)) return r;
+      cudaFuncAttributes fa;
+      EG_CUDA(cudaFuncGetAttributes(&fa, func));
+    }
   }
   return 0;
 }
