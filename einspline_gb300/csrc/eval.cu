@@ -1348,6 +1348,12 @@ static int num_sms() {
 // set_tile.
 void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) {
   if (t->tile_tx || a.npts <= 0) return;
+  if (a.npts == 1) {
+    // what the search below finds, without its 0.3 us
+    tx = 32;
+    ty = pb = 1;
+    return;
+  }
   EvalArgs b = a;
   const void *func;
   dim3 block;
@@ -1508,8 +1514,13 @@ static double row_reuse(const Table *t, int64_t npts) {
 //                  64^3 x 1024 12,000 (2.8)            328 / 335
 //                  64^3 x 256 complex 16,384 (3.6)     219 / 208
 //                  64^3 x 1024 60,000 (13)             1521 / 1230
+// A launch of a few points is one chain of loads, of which the pipeline has
+// more in flight: 24^3 x 1024, 1 to 16 points 3.9 / 4.3, 48 points 5.1 / 4.9;
+// 45^3 x 203, 100 points 4.8 / 5.0.
 constexpr size_t kL2Table = 112u << 20, kNearL2Table = 300u << 20;
+constexpr int64_t kDirectEvals = 20000;
 static bool direct_pays(const Table *t, bool sorted, int64_t npts) {
+  if (npts * t->ncol < kDirectEvals) return false;
   if (t->table_bytes < kL2Table) return true;
   return sorted && (t->table_bytes < kNearL2Table || row_reuse(t, npts) >= 3.0);
 }
