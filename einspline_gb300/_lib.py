@@ -115,6 +115,12 @@ class DetOpts(C.Structure):
                 ("pos_f64", C.c_int), ("rule", C.c_int)]
 
 
+class DetBatch(C.Structure):
+    _fields_ = [("a", C.c_void_p), ("a_step", C.c_int64), ("a_count", C.c_int64),
+                ("ainv", C.c_void_p), ("ainv_step", C.c_int64), ("ainv_count", C.c_int64),
+                ("rows", C.c_void_p), ("row_step", C.c_int64), ("row_count", C.c_int64)]
+
+
 class TableInfo(C.Structure):
     _fields_ = [("kind", C.c_int), ("storage", C.c_int), ("num_splines", C.c_int), ("ncol", C.c_int),
                 ("ncol_pad", C.c_int), ("elem_bytes", C.c_int), ("nx", C.c_int), ("ny", C.c_int),
@@ -221,6 +227,8 @@ def _signatures():
     sig["einspline_gb300_fill_uniform"] = ([vp, i64, i32, C.c_uint64, i64, dbl, dbl, vp], i32)
     sig["einspline_gb300_det_ratio"] = ([vp, C.POINTER(DetOpts), i32, vp, vp, vp, vp, vp, vp, vp], i32)
     sig["einspline_gb300_det_update"] = ([C.POINTER(DetOpts), i32, vp, vp, vp, vp, vp], i32)
+    sig["einspline_gb300_det_update_accepted"] = ([C.POINTER(DetOpts), i32, vp, C.POINTER(DetBatch), vp, vp, vp, vp],
+                                                  i32)
     sig["einspline_gb300_server_create"] = ([vp, C.POINTER(ServerOpts)], vp)
     sig["einspline_gb300_server_destroy"] = ([vp], i32)
     sig["einspline_gb300_server_submit"] = ([vp, vp, i32], i64)

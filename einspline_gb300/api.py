@@ -661,6 +661,11 @@ class Determinants:
         self.W, self.ld = int(A.shape[0]), int(ainv.shape[-1])
         self.nelec, self.trans = int(nelec), int(trans)
         self._cache = {}
+        self._status = None
+        if A.is_cuda:
+            self._status = _status_words.pop() if _status_words else torch.zeros(1, dtype=torch.int32).pin_memory()
+            self._refused = C.c_int.from_address(self._status.data_ptr())
+            self._refused.value = 0
         self.a_ptrs = self._ptrs(A)
         self.ainv_ptrs = self._ptrs(ainv)
         self.work = torch.empty(2 * self.nelec * self.W, dtype=torch.float32, device=A.device)
@@ -716,20 +721,40 @@ class Determinants:
 
     def update(self, k: int, accepted, rows, stream=None):
         """Sherman-Morrison update of the accepted walkers (indices) whose
-        row k becomes rows[i] (rows: [W, >= nelec] float32 CUDA tensor)."""
+        row k becomes rows[i] (rows: [W, >= nelec] float32 CUDA tensor).
+        An index out of range refuses the whole call on the GPU; the next
+        call raises IndexError for it."""
         torch = _torch()
         idx = self._index(accepted)
         n = int(idx.numel())
+        self._raise_refused()
         if n == 0:
             return
-        a = self.a_ptrs[idx].contiguous()
-        ai = self.ainv_ptrs[idx].contiguous()
-        r = self._ptrs(rows)[idx].contiguous()
-        o = self.opts(k)
-        s = C.c_void_p(stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream)
-        _lib().einspline_gb300_det_update(C.byref(o), n, C.c_void_p(a.data_ptr()), C.c_void_p(ai.data_ptr()),
-                                          C.c_void_p(r.data_ptr()), C.c_void_p(self.work.data_ptr()), s)
+        idx = idx.contiguous()
+        scratch = torch.empty(3 * n + 1, dtype=torch.int64, device=self.A.device)
+        if stream is not None:
+            scratch.record_stream(stream)
+            idx.record_stream(stream)
+        at = lambda t: (t.data_ptr(), t.stride(0) * t.element_size(), t.shape[0])  # noqa: E731
+        o, b = self.opts(k), L.DetBatch(*at(self.A), *at(self.ainv), *at(rows))
+        s = stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream
+        _lib().einspline_gb300_det_update_accepted(C.byref(o), n, idx.data_ptr(), C.byref(b), self.work.data_ptr(),
+                                                   scratch.data_ptr(), self._status.data_ptr(), s)
         check()
+
+    def _raise_refused(self):
+        if self._refused.value:
+            self._refused.value = 0
+            raise IndexError("Determinants.update: an earlier call's walker index was out of range; "
+                             "it updated nothing")
+
+    def __del__(self):
+        # kept for the next object: a launch that refuses may still write it
+        if getattr(self, "_status", None) is not None:
+            _status_words.append(self._status)
+
+
+_status_words = []  # pinned words of objects that are gone
 
 
 def launch_count() -> int:

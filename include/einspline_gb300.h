@@ -372,6 +372,26 @@ int einspline_gb300_det_ratio(einspline_gb300_table *t, const einspline_gb300_de
 int einspline_gb300_det_update(const einspline_gb300_det_opts *opts, int naccept, float *const *a_d,
                                float *const *ainv_d, const float *const *row_d, float *work_d, void *stream);
 
+/* The same for walkers held at a fixed distance from each other, by index:
+ * walker w's A, inverse and new row are at a + w * a_step and so on (steps in
+ * bytes, counts of walkers there).  accepted_d: naccept distinct walker
+ * indices in device memory; a negative one counts from the end.  ptrs_d:
+ * device scratch of 3 * naccept + 1 int64; work_d as above.  An index outside
+ * a count refuses the whole call on the device: nothing is updated, and
+ * *status (NULL, or an int the device can write, such as pinned host memory)
+ * becomes 1.  Two launches on stream, no copy. */
+typedef struct {
+  float *a;
+  int64_t a_step, a_count;
+  float *ainv;
+  int64_t ainv_step, ainv_count;
+  const float *rows;
+  int64_t row_step, row_count;
+} einspline_gb300_det_batch;
+int einspline_gb300_det_update_accepted(const einspline_gb300_det_opts *opts, int naccept, const int64_t *accepted_d,
+                                        const einspline_gb300_det_batch *batch, float *work_d, int64_t *ptrs_d,
+                                        int *status, void *stream);
+
 /* FP64 (d and z) tables: how evaluations compute.
  *   0 (default): IEEE FP64 fused multiply-adds.  On GB300 the FP64 pipe is a
  *     small fraction of the FP32 one, and this path is bound by it, far below
