@@ -30,6 +30,18 @@ def _torch():
     return torch
 
 
+def _stream(torch, stream):
+    """Handle of stream, or of the current device's current one (as
+    torch.cuda.current_stream gives it, without a Stream object per call)."""
+    if stream is not None:
+        return stream.cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def _addr(t):
+    return t.data_ptr() if t is not None else None
+
+
 def out_dtype(kind):
     return np.float32 if kind in "sc" else np.float64
 
@@ -261,18 +273,16 @@ class MultiUBspline3D:
         float32/float64.  Returns (vals, grads, hess) torch tensors."""
         torch = _torch()
         P = int(pos.shape[0])
-        dt = torch.float32 if self.kind in "sc" else torch.float64
         if out is None:
+            dt = torch.float32 if self.kind in "sc" else torch.float64
             shp = self.out_shapes(P, layout)
             out = (torch.empty(shp[0], dtype=dt, device=pos.device),
                    torch.empty(shp[1], dtype=dt, device=pos.device) if vgh else None,
                    torch.empty(shp[2], dtype=dt, device=pos.device) if vgh else None)
         o = self.opts(vgh, pos.dtype == torch.float64, rule, layout, sort)
-        ptr = lambda t: C.c_void_p(t.data_ptr()) if t is not None else C.c_void_p(0)  # noqa: E731
-        s = C.c_void_p(stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream)
-        _lib().einspline_gb300_eval_3d(self.table, C.byref(o), P, ptr(pos), ptr(out[0]), ptr(out[1]),
-                                       ptr(out[2]), s)
-        check()
+        if _lib().einspline_gb300_eval_3d(self.table, C.byref(o), P, pos.data_ptr(), _addr(out[0]), _addr(out[1]),
+                                          _addr(out[2]), _stream(torch, stream)):
+            check()
         return out
 
     def set_fp64_mode(self, mode: int) -> None:
@@ -712,11 +722,10 @@ class Determinants:
         lapl = torch.empty(W, dtype=torch.float32, device=dev) if grad_lapl else None
         row_ptrs = self._ptrs(rows) if rows is not None else None
         o = self.opts(k, pos.dtype == torch.float64, rule)
-        ptr = lambda t: C.c_void_p(t.data_ptr()) if t is not None else C.c_void_p(0)  # noqa: E731
-        s = C.c_void_p(stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream)
-        _lib().einspline_gb300_det_ratio(spline.table, C.byref(o), W, ptr(pos), ptr(self.ainv_ptrs), ptr(ratio),
-                                         ptr(grad), ptr(lapl), ptr(row_ptrs), s)
-        check()
+        if _lib().einspline_gb300_det_ratio(spline.table, C.byref(o), W, pos.data_ptr(), self.ainv_ptrs.data_ptr(),
+                                            ratio.data_ptr(), _addr(grad), _addr(lapl), _addr(row_ptrs),
+                                            _stream(torch, stream)):
+            check()
         return ratio, grad, lapl
 
     def update(self, k: int, accepted, rows, stream=None):
@@ -737,10 +746,10 @@ class Determinants:
             idx.record_stream(stream)
         at = lambda t: (t.data_ptr(), t.stride(0) * t.element_size(), t.shape[0])  # noqa: E731
         o, b = self.opts(k), L.DetBatch(*at(self.A), *at(self.ainv), *at(rows))
-        s = stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream
-        _lib().einspline_gb300_det_update_accepted(C.byref(o), n, idx.data_ptr(), C.byref(b), self.work.data_ptr(),
-                                                   scratch.data_ptr(), self._status.data_ptr(), s)
-        check()
+        if _lib().einspline_gb300_det_update_accepted(C.byref(o), n, idx.data_ptr(), C.byref(b),
+                                                      self.work.data_ptr(), scratch.data_ptr(),
+                                                      self._status.data_ptr(), _stream(torch, stream)):
+            check()
 
     def _raise_refused(self):
         if self._refused.value:
