@@ -1224,7 +1224,11 @@ int einspline_gb300_det_ratio(einspline_gb300_table *t, const einspline_gb300_de
     // for each inverse entry.
     const int tiles = (d.n + 127) / 128;
     const int64_t wave = kDtBlocksPerSM * (int64_t)num_sms();
-    const int pb = (int)std::min<int64_t>(kDtMaxWalkers, std::max<int64_t>(std::max(1, kDtUnits / tiles), nwalkers / (4 * wave)));
+    // Few walkers spread over the SMs, three blocks each, before blocks get
+    // longer: N = 128, 4 to 48 walkers 8.8 / 4.4, 200 walkers 9.0 / 5.6.
+    int64_t units = std::max(1, kDtUnits / tiles);
+    if (nwalkers <= 2 * wave) units = std::min<int64_t>(units, (nwalkers + 3 * num_sms() - 1) / (3 * num_sms()));
+    const int pb = (int)std::min<int64_t>(kDtMaxWalkers, std::max<int64_t>(units, nwalkers / (4 * wave)));
     d.e.pb = pb;
     const unsigned grid = (unsigned)((nwalkers + pb - 1) / pb);
     EG_CUDA(t->storage == ST_F16 ? launch_det_tc<ST_F16>(d, gl, grid, s) : launch_det_tc<ST_BF16>(d, gl, grid, s));
