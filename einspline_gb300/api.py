@@ -673,7 +673,10 @@ class Determinants:
         self._cache = {}
         self._status = None
         if A.is_cuda:
-            self._status = _status_words.pop() if _status_words else torch.zeros(1, dtype=torch.int32).pin_memory()
+            try:
+                self._status = _status_words.pop()
+            except IndexError:
+                self._status = torch.zeros(1, dtype=torch.int32).pin_memory()
             self._refused = C.c_int.from_address(self._status.data_ptr())
             self._refused.value = 0
         self.a_ptrs = self._ptrs(A)
@@ -759,7 +762,7 @@ class Determinants:
 
     def __del__(self):
         # kept for the next object: a launch that refuses may still write it
-        if getattr(self, "_status", None) is not None:
+        if getattr(self, "_status", None) is not None and _status_words is not None:
             _status_words.append(self._status)
 
 
