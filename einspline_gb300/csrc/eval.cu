@@ -281,6 +281,45 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
   }
 }
 
+// The points and columns a thread of the wide value kernel, or of the FP64 vgh
+// kernel, goes through.  A full tile has a thread for each VW columns of a
+// point.  The last tile of a
+// table whose columns do not fill it (777 columns in tiles of 256 leave 9) has
+// fewer columns than threads: there the (point, columns) pairs of the block's
+// points are dealt to all threads in turn.  I16 56 x 60 x 52 x 777, 24,000
+// points: 264 -> 235 us (7 of these by decode2).  FP64 vgh, whose pipe takes
+// as long for an idle lane: complex 32 x 9 x 23 x 8, 12,392 points: 527 ->
+// 161 us; 40^3 x 203 real, 8000 points: 1142 -> 994.  The other kernels
+// do not deal: their tiles are narrower, or in vgh a block-wide point index is
+// worth the 2-5 % that a thread's own costs.
+struct ColumnWalk {
+  int point, lane, lanes, dp, dl;
+  // cols columns left for a tile of width threads, dealt to thread tid of nthr
+  __device__ __forceinline__ ColumnWalk(int cols, int width, int vw, int tid, int nthr) {
+    lanes = min(width, (cols + vw - 1) / vw);
+    point = tid / lanes;
+    lane = tid - point * lanes;
+    dp = nthr / lanes;
+    dl = nthr - dp * lanes;
+  }
+  __device__ __forceinline__ void next() {
+    point += dp;
+    lane += dl;
+    if (lane >= lanes) {
+      lane -= lanes;
+      point++;
+    }
+  }
+  // (point, columns) pairs this thread, at its first, has of pn points'
+  __device__ __forceinline__ int count(int pn) const {
+    const int n = pn * lanes - (point * lanes + lane), step = dp * lanes + dl;
+    return n > 0 ? (n + step - 1) / step : 0;
+  }
+};
+
+// Direct-load kernels that deal their pairs.
+static constexpr bool deals(int st, bool vgh) { return st == ST_F64 && vgh; }
+
 template <int ST, bool VGH, bool SHIFT>
 __global__ void __launch_bounds__(256) k_eval(const EvalArgs a) {
   using A = typename CT<ST>::A;
@@ -338,10 +377,22 @@ __global__ void __launch_bounds__(256) k_eval(const EvalArgs a) {
     }
   }
 
+  const int64_t xsb = a.xs * CT<ST>::BYTES, ysb = a.ys * CT<ST>::BYTES, zsb = a.zs * CT<ST>::BYTES;
+  if constexpr (deals(ST, VGH)) {
+    const int c_first = tile * blockDim.x * VW;
+    for (ColumnWalk it(a.ncol - c_first, blockDim.x, VW, tid, nthr); it.point < pn; it.next()) {
+      const int pp = it.point, col0 = c_first + it.lane * VW;
+      const char *base = reinterpret_cast<const char *>(a.coefs) + (int64_t)col0 * CT<ST>::BYTES +
+                         sidx[3 * pp] * xsb + sidx[3 * pp + 1] * ysb + sidx[3 * pp + 2] * zsb;
+      A o[10][VW];
+      contract<ST, VGH>(base, xsb, ysb, zsb, sw + pp * 36, o);
+      epilogue<A, VW, VGH>(a, ssrc[pp], col0, o);
+    }
+    return;
+  }
   const int col0 = (tile * blockDim.x + threadIdx.x) * VW;
   if (col0 >= a.ncol) return;
   const char *cbase = reinterpret_cast<const char *>(a.coefs) + (int64_t)col0 * CT<ST>::BYTES;
-  const int64_t xsb = a.xs * CT<ST>::BYTES, ysb = a.ys * CT<ST>::BYTES, zsb = a.zs * CT<ST>::BYTES;
   for (int pp = threadIdx.y; pp < pn; pp += blockDim.y) {
     const char *base = cbase + sidx[3 * pp] * xsb + sidx[3 * pp + 1] * ysb + sidx[3 * pp + 2] * zsb;
     A o[10][VW];
@@ -358,38 +409,6 @@ __global__ void __launch_bounds__(256) k_eval(const EvalArgs a) {
     }
   }
 }
-
-// The points and columns a thread of the wide value kernel goes through.  A
-// full tile has a thread for each VW columns of a point.  The last tile of a
-// table whose columns do not fill it (777 columns in tiles of 256 leave 9) has
-// fewer columns than threads: there the (point, columns) pairs of the block's
-// points are dealt to all threads in turn.  I16 56 x 60 x 52 x 777, 24,000
-// points: 264 -> 235 us (7 of these by decode2).  The other pipelined kernels
-// do not deal: their tiles are narrower, or in vgh a block-wide point index is
-// worth the 2-5 % that a thread's own costs.
-struct ColumnWalk {
-  int point, lane, lanes, dp, dl;
-  __device__ __forceinline__ ColumnWalk(int cols, int nthr, int vw) {
-    lanes = min(nthr, (cols + vw - 1) / vw);
-    point = threadIdx.x / lanes;
-    lane = threadIdx.x - point * lanes;
-    dp = nthr / lanes;
-    dl = nthr - dp * lanes;
-  }
-  __device__ __forceinline__ void next() {
-    point += dp;
-    lane += dl;
-    if (lane >= lanes) {
-      lane -= lanes;
-      point++;
-    }
-  }
-  // (point, columns) pairs this thread, at its first, has of pn points'
-  __device__ __forceinline__ int count(int pn) const {
-    const int n = pn * lanes - (point * lanes + lane), step = dp * lanes + dl;
-    return n > 0 ? (n + step - 1) / step : 0;
-  }
-};
 
 // Pipelined variant: a stage is one x-plane (16 stencil rows) of one point.
 // Each thread copies its own columns of the rows of stage s+2 into shared
@@ -425,7 +444,7 @@ __device__ __forceinline__ void eval_pipe_body(const EvalArgs &a) {
   int col0 = (tile * blockDim.x + threadIdx.x) * VW, S = pn * 4;
   const int c_first = tile * nthr * VW;
   // dealt: the pair this thread copies and, behind it, the one it reduces
-  ColumnWalk in(DEAL ? a.ncol - c_first : 1, nthr, VW), it = in;
+  ColumnWalk in(DEAL ? a.ncol - c_first : 1, nthr, VW, threadIdx.x, nthr), it = in;
   if constexpr (DEAL) S = in.count(pn) * 4;
   else if (col0 >= a.ncol) return;
   const char *cbase = reinterpret_cast<const char *>(a.coefs) + (int64_t)(DEAL ? c_first : col0) * CT<ST>::BYTES;
@@ -1365,18 +1384,41 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   const int64_t wave = b.mode == 5 ? kTcBlocksPerSM * sms : resident_blocks(func, (int)(block.x * block.y), smem);
   const int64_t per = wave / sms;
   if (per < 1) return;
+  // points a block works on at once, and rounds it takes for p points
+  const int need = (t->ncol + elems_per_thread(t) - 1) / elems_per_thread(t);
+  const bool deal = b.mode == 0 && deals(kernel_storage(t), vgh);
+  auto at_once = [&](int x, int y) { return deal ? std::min(pb, x * y / std::min(x, need)) : y; };
+  auto rounds = [&](int x, int y, int p) { return deal ? (p * std::min(x, need) + x * y - 1) / (x * y) : p / y; };
   // Values by direct loads hide their latency only behind other warps, and
   // their blocks start quickly: one point a lane below four waves of the given
   // blocks (FP32, 40^3 x 1000, 3000 points: 86 against 99 us; from five
   // waves on, 4 points a lane are up to 10 % faster), for FP64, which its
   // arithmetic bounds, below one.
-  if (b.mode == 0 && (!vgh || t->storage == ST_F64) && (a.npts + pb - 1) / pb * b.ntiles < (t->storage == ST_F64 ? 1 : 4) * wave) pb = (int)block.y;
+  if (b.mode == 0 && (!vgh || t->storage == ST_F64) && (a.npts + pb - 1) / pb * b.ntiles < (t->storage == ST_F64 ? 1 : 4) * wave) pb = at_once((int)block.x, (int)block.y);
   // groups' blocks; the wide value kernel deals the columns of a ragged last
   // tile to all its threads, so that tile counts by its share of the columns
   const bool dealt = b.mode == 3 && !vgh;
   const int64_t tcols = (int64_t)tx * elems_per_thread(t) * 2;
   auto blocks_of = [&](int64_t groups) { return dealt ? (groups * a.ncol + tcols - 1) / tcols : groups * b.ntiles; };
   const int64_t full = (a.npts + pb - 1) / pb * b.ntiles;
+  if (full >= wave && deal) {
+    // up to four waves, whose blocks all take as long: the size with the
+    // least rounds on the fullest SM (30^3 x 64, 12,392 points: 520 us with 16
+    // points a block, 463 so); beyond them the launch's tail of short blocks
+    // evens it out
+    if (full >= 4 * wave) return;
+    const int x = (int)block.x, y = (int)block.y, p0 = pb;
+    int64_t least = INT64_MAX;
+    for (int r = rounds(x, y, p0); r >= 1; r--) {
+      const int p = std::max(1, std::min(p0, r * x * y / std::min(x, need)));
+      const int64_t cost = ((a.npts + p - 1) / p * b.ntiles + sms - 1) / sms * rounds(x, y, p);
+      if (cost < least) {
+        least = cost;
+        pb = p;
+      }
+    }
+    return;
+  }
   if (full >= wave) {
     // between one and two waves of the copy pipelines' blocks: the size whose
     // whole waves take the least points one after another (FP32 48^3 x 400,
@@ -1402,10 +1444,11 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
     const int64_t tiles = fixed ? b.ntiles : ((int64_t)b.ntiles * width + x - 1) / x;
     for (int y = lanes; y >= 1; y /= 2) {
       const int64_t fit = fixed ? per : std::min<int64_t>(32, per * width * lanes / (x * y));
-      for (int p = y; p <= pb; p += y) {
+      const int u = at_once(x, y);
+      for (int p = u; p <= pb; p += u) {
         const int64_t blocks = (a.npts + p - 1) / p * tiles, deep = (blocks + sms - 1) / sms;
         if (deep > fit) continue;
-        const int64_t work = deep * p * x, chain = p / y;
+        const int64_t chain = rounds(x, y, p), work = deep * chain * x * y;
         if (work < best_work || (work == best_work && chain < best_chain)) {
           best_work = work;
           best_chain = chain;
@@ -1586,7 +1629,7 @@ void pick_tile(Table *t, bool vgh, int64_t npts, int &tx, int &ty, int &pb, bool
   if (kernel_storage(t) == ST_F64 && vgh) {
     if (tx > 128) tx = 128;
     ty = std::min(8, 128 / tx);
-    pb = 4 * ty;
+    pb = std::min(64, 4 * tx * ty / std::min(tx, need));
     return;
   }
   if (!vgh && t->storage == ST_F32 && t->tile_mode <= 0) {
