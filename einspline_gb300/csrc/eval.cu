@@ -281,15 +281,15 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
   }
 }
 
-// The points and columns a thread of the wide value kernel, or of the FP64 vgh
-// kernel, goes through.  A full tile has a thread for each VW columns of a
+// The points and columns a thread of the wide value kernel, or of the FP64
+// direct-load kernels, goes through.  A full tile has a thread for each VW columns of a
 // point.  The last tile of a
 // table whose columns do not fill it (777 columns in tiles of 256 leave 9) has
 // fewer columns than threads: there the (point, columns) pairs of the block's
 // points are dealt to all threads in turn.  I16 56 x 60 x 52 x 777, 24,000
-// points: 264 -> 235 us (7 of these by decode2).  FP64 vgh, whose pipe takes
-// as long for an idle lane: complex 32 x 9 x 23 x 8, 12,392 points: 527 ->
-// 161 us; 40^3 x 203 real, 8000 points: 1142 -> 994.  The other kernels
+// points: 264 -> 235 us (7 of these by decode2).  FP64, whose pipe takes
+// as long for an idle lane: complex 32 x 9 x 23 x 8, 12,392 points vgh: 527 ->
+// 161 us; 40^3 x 203 real, 8000 points: 1142 -> 994, values 332 -> 297.  The other kernels
 // do not deal: their tiles are narrower, or in vgh a block-wide point index is
 // worth the 2-5 % that a thread's own costs.
 struct ColumnWalk {
@@ -318,7 +318,7 @@ struct ColumnWalk {
 };
 
 // Direct-load kernels that deal their pairs.
-static constexpr bool deals(int st, bool vgh) { return st == ST_F64 && vgh; }
+static constexpr bool deals(int st) { return st == ST_F64; }
 
 template <int ST, bool VGH, bool SHIFT>
 __global__ void __launch_bounds__(256) k_eval(const EvalArgs a) {
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(256) k_eval(const EvalArgs a) {
   }
 
   const int64_t xsb = a.xs * CT<ST>::BYTES, ysb = a.ys * CT<ST>::BYTES, zsb = a.zs * CT<ST>::BYTES;
-  if constexpr (deals(ST, VGH)) {
+  if constexpr (deals(ST)) {
     const int c_first = tile * blockDim.x * VW;
     for (ColumnWalk it(a.ncol - c_first, blockDim.x, VW, tid, nthr); it.point < pn; it.next()) {
       const int pp = it.point, col0 = c_first + it.lane * VW;
@@ -1386,7 +1386,7 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   if (per < 1) return;
   // points a block works on at once, and rounds it takes for p points
   const int need = (t->ncol + elems_per_thread(t) - 1) / elems_per_thread(t);
-  const bool deal = b.mode == 0 && deals(kernel_storage(t), vgh);
+  const bool deal = b.mode == 0 && deals(kernel_storage(t));
   auto at_once = [&](int x, int y) { return deal ? std::min(pb, x * y / std::min(x, need)) : y; };
   auto rounds = [&](int x, int y, int p) { return deal ? (p * std::min(x, need) + x * y - 1) / (x * y) : p / y; };
   // Values by direct loads hide their latency only behind other warps, and
@@ -1643,6 +1643,7 @@ void pick_tile(Table *t, bool vgh, int64_t npts, int &tx, int &ty, int &pb, bool
   ty = 256 / tx;
   if (ty > 8) ty = 8;
   pb = 2 * ty;
+  if (kernel_storage(t) == ST_F64) pb = std::min(64, 2 * tx * ty / std::min(tx, need));
 }
 
 int wait_status(Table *t, const char *fn) {

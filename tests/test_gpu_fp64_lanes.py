@@ -35,3 +35,20 @@ def test_dealt_columns(kind, N):
         G.set_tile(tx, ty, pb)
         for a, b in zip(G.eval(pos), ref):
             assert torch.equal(a, b), (tx, ty, pb)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,N", [("d", 1), ("d", 3), ("z", 8), ("d", 64), ("d", 203), ("z", 257)])
+def test_dealt_values(kind, N):
+    torch = pytest.importorskip("torch")
+    G = api.MultiUBspline3D(kind, GRID, [(api.PERIODIC, api.PERIODIC)] * 3, N)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(N)
+    G.set_device(0, torch.rand((N,) + G.M + ((2,) if kind == "z" else ()), generator=g, device="cuda",
+                               dtype=torch.float64) - 0.5)
+    G.flush()
+    pos = torch.rand((9001, 3), generator=g, device="cuda", dtype=torch.float64)
+    ref = G.eval(pos, vgh=False)[0]
+    assert torch.equal(ref, G.eval(pos)[0])
+    for n in (1, 2, 17, 64, 65, 300, 3001):
+        assert torch.equal(G.eval(pos[:n], vgh=False)[0], ref[:n]), n
