@@ -795,7 +795,7 @@ int einspline_gb300_autotune(einspline_gb300_table *t, int64_t npts, int vgh) {
   if (npts < 1) return fail(EINSPLINE_GB300_EINVAL, "npts must be >= 1");
   if (int r = table_flush(t)) return r;
   const size_t rb = t->storage == ST_F64 ? 8 : 4;
-  const size_t out_b = (size_t)npts * t->ncol * rb * (vgh ? 10 : 1);
+  const size_t out_b = align_up_sz((size_t)npts * t->ncol * rb * (vgh ? 10 : 1), 256);  // doubles follow
   void *buf = nullptr;
   if (cudaMalloc(&buf, out_b + (size_t)npts * 24) != cudaSuccess) {
     cudaGetLastError();
