@@ -671,7 +671,7 @@ class Determinants:
         self.W, self.ld = int(A.shape[0]), int(ainv.shape[-1])
         self.nelec, self.trans = int(nelec), int(trans)
         self._cache = {}
-        self._status = None
+        self._status = self._refused = None  # host tensors: nothing runs that could refuse
         if A.is_cuda:
             try:
                 self._status = _status_words.pop()
@@ -751,11 +751,11 @@ class Determinants:
         o, b = self.opts(k), L.DetBatch(*at(self.A), *at(self.ainv), *at(rows))
         if _lib().einspline_gb300_det_update_accepted(C.byref(o), n, idx.data_ptr(), C.byref(b),
                                                       self.work.data_ptr(), scratch.data_ptr(),
-                                                      self._status.data_ptr(), _stream(torch, stream)):
+                                                      _addr(self._status), _stream(torch, stream)):
             check()
 
     def _raise_refused(self):
-        if self._refused.value:
+        if self._refused is not None and self._refused.value:
             self._refused.value = 0
             raise IndexError("Determinants.update: an earlier call's walker index was out of range; "
                              "it updated nothing")

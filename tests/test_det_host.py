@@ -1,0 +1,31 @@
+"""Determinants over host tensors: the object works as far as no kernel runs."""
+import pytest
+
+from einspline_gb300 import api
+
+
+def population(torch, W=3, n=4):
+    A = torch.eye(n).repeat(W, 1, 1)
+    return api.Determinants(A, A.clone(), n), A[:, 1].contiguous()
+
+
+@pytest.mark.parametrize("none", [[], ()])
+def test_no_accepted_walker_updates_nothing(none):
+    torch = pytest.importorskip("torch")
+    D, rows = population(torch)
+    assert D.update(1, none, rows) is None
+    assert D.update(1, torch.zeros(0, dtype=torch.int32), rows) is None
+
+
+def test_update_reaches_the_library(monkeypatch):
+    torch = pytest.importorskip("torch")
+    D, rows = population(torch)
+
+    class Lib:
+        def einspline_gb300_det_update_accepted(self, o, n, idx, batch, work, scratch, status, stream):
+            assert n == 2 and idx and work and scratch and not status and stream == 5
+            return 0
+
+    monkeypatch.setattr(api, "_lib", Lib)
+    monkeypatch.setattr(api, "_stream", lambda torch, stream: 5)
+    D.update(1, [0, 2], rows)
