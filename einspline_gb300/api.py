@@ -734,6 +734,8 @@ class Determinants:
     def update(self, k: int, accepted, rows, stream=None):
         """Sherman-Morrison update of the accepted walkers (indices) whose
         row k becomes rows[i] (rows: [W, >= nelec] float32 CUDA tensor).
+        For a stream other than the current one, the matrices and rows have
+        to be ready there, and accepted, if a tensor, on the current one.
         An index out of range refuses the whole call on the GPU; the next
         call raises IndexError for it."""
         torch = _torch()
@@ -743,10 +745,18 @@ class Determinants:
         if n == 0:
             return
         idx = idx.contiguous()
-        scratch = torch.empty(3 * n + 1, dtype=torch.int64, device=self.A.device)
-        if stream is not None:
-            scratch.record_stream(stream)
+        if stream is None or stream == torch.cuda.current_stream(self.A.device):
+            scratch = torch.empty(3 * n + 1, dtype=torch.int64, device=self.A.device)
+        else:
+            # the scratch is the stream's own memory, what the current stream
+            # still does to the indices comes first, and the stream may go on
+            # using them and the work space after they are dropped here
+            if isinstance(accepted, torch.Tensor):
+                stream.wait_stream(torch.cuda.current_stream(self.A.device))
+            with torch.cuda.stream(stream):
+                scratch = torch.empty(3 * n + 1, dtype=torch.int64, device=self.A.device)
             idx.record_stream(stream)
+            self.work.record_stream(stream)
         at = lambda t: (t.data_ptr(), t.stride(0) * t.element_size(), t.shape[0])  # noqa: E731
         o, b = self.opts(k), L.DetBatch(*at(self.A), *at(self.ainv), *at(rows))
         if _lib().einspline_gb300_det_update_accepted(C.byref(o), n, idx.data_ptr(), C.byref(b),

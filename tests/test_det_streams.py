@@ -46,9 +46,6 @@ def test_update_on_another_stream_is_ordered(monkeypatch, kind):
     A = torch.eye(4).repeat(3, 1, 1)
     rows = A[:, 1].contiguous()
     D = api.Determinants(A, A.clone(), 4)
-    if not hasattr(D, "_refused"):
-        D._refused = D._status = torch.zeros(1, dtype=torch.int32)
-        D._refused = type("Word", (), {"value": 0})()
     s = Recorder(torch, monkeypatch)
     idx = [0, 2] if kind == "list" else torch.tensor([0, 2], dtype=getattr(torch, kind))
     D.update(1, idx, rows, stream=s)
