@@ -745,6 +745,8 @@ class Determinants:
         if n == 0:
             return
         idx = idx.contiguous()
+        if stream is not None and not isinstance(stream, torch.cuda.Stream):
+            stream = torch.cuda.ExternalStream(stream.cuda_stream)  # another library's
         if stream is None or stream == torch.cuda.current_stream(self.A.device):
             scratch = torch.empty(3 * n + 1, dtype=torch.int64, device=self.A.device)
         else:

@@ -27,6 +27,7 @@ class Recorder:
         monkeypatch.setattr(torch, "empty", logged_empty)
         monkeypatch.setattr(torch.cuda, "stream", on)
         monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: "current")
+        monkeypatch.setattr(torch.cuda, "Stream", Recorder)
         monkeypatch.setattr(torch.Tensor, "record_stream", lambda t, s: self.log.append(("keep", t.data_ptr(), s)))
         monkeypatch.setattr(api, "_lib", lambda: self)
 
@@ -59,6 +60,21 @@ def test_update_on_another_stream_is_ordered(monkeypatch, kind):
     assert (("wait", "current") in before) == (kind != "list")
     # indices and work space stay until the stream is done with them
     assert ("keep", launch[1], s) in s.log and ("keep", launch[2], s) in s.log
+
+
+def test_stream_of_another_library(monkeypatch):
+    """An object with a cuda_stream handle is a stream, as for the other calls."""
+    torch = pytest.importorskip("torch")
+    A = torch.eye(4).repeat(3, 1, 1)
+    rows = A[:, 1].contiguous()
+    D = api.Determinants(A, A.clone(), 4)
+    s = Recorder(torch, monkeypatch)
+    s.cuda_stream = 11
+    monkeypatch.setattr(torch.cuda, "ExternalStream", lambda handle: s if handle == 11 else None)
+    foreign = type("Foreign", (), {"cuda_stream": 11})()
+    D.update(1, [0, 2], rows, stream=foreign)
+    (launch,) = [e for e in s.log if e[0] == "launch"]
+    assert launch[3] == 11 and ("alloc", s) in s.log and ("keep", launch[1], s) in s.log
 
 
 @pytest.mark.gpu
