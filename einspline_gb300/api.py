@@ -744,6 +744,8 @@ class Determinants:
         self._raise_refused()
         if n == 0:
             return
+        if rows.device != self.A.device:
+            raise RuntimeError(f"Determinants.update: rows are on {rows.device}, the matrices on {self.A.device}")
         idx = idx.contiguous()
         if stream is not None and not isinstance(stream, torch.cuda.Stream):
             stream = torch.cuda.ExternalStream(stream.cuda_stream)  # another library's

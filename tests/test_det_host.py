@@ -29,3 +29,15 @@ def test_update_reaches_the_library(monkeypatch):
     monkeypatch.setattr(api, "_lib", Lib)
     monkeypatch.setattr(api, "_stream", lambda torch, stream: 5)
     D.update(1, [0, 2], rows)
+
+
+def test_rows_of_another_device_are_refused(monkeypatch):
+    """Their addresses would otherwise reach a kernel of the matrices' device."""
+    torch = pytest.importorskip("torch")
+    D, _ = population(torch)
+    called = []
+    monkeypatch.setattr(api, "_lib", lambda: called.append(1))
+    monkeypatch.setattr(api, "_stream", lambda torch, stream: 5)
+    with pytest.raises(RuntimeError):
+        D.update(1, [0, 2], torch.empty((3, 4), device="meta"))
+    assert not called
