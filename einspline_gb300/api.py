@@ -701,14 +701,27 @@ class Determinants:
             return self._remember(key, base + t.data_ptr())
         return self._cache[key]
 
-    def _index(self, accepted):
+    def _index(self, accepted, count):
+        """accepted as int64 on the matrices' device.  Indices that the host
+        holds are checked here: -count <= index < count."""
         torch = _torch()
         if isinstance(accepted, torch.Tensor):
+            if accepted.device.type == "cpu" and accepted.numel():
+                accepted = accepted.to(torch.int64)
+                self._in_range(int(accepted.min()), int(accepted.max()), count)
             return accepted.to(device=self.A.device, dtype=torch.int64)
         key = ("i", tuple(int(i) for i in accepted))
+        if key[1]:
+            self._in_range(min(key[1]), max(key[1]), count)
         if key not in self._cache:
             return self._remember(key, torch.as_tensor(key[1], dtype=torch.int64, device=self.A.device))
         return self._cache[key]
+
+    @staticmethod
+    def _in_range(lo, hi, count):
+        if lo < -count or hi >= count:
+            raise IndexError(f"Determinants.update: walker index {lo if lo < -count else hi} is out of range for "
+                             f"{count} walkers")
 
     def opts(self, k, pos_f64=False, rule=1):
         return L.DetOpts(self.nelec, int(k), self.ld, self.trans, int(pos_f64), int(rule))
@@ -716,8 +729,10 @@ class Determinants:
     def ratio(self, spline: "MultiUBspline3D", pos, k: int, grad_lapl=True, rows=None, rule=1, stream=None):
         """Ratios (and gradient / Laplacian ratios) of every walker moving
         electron k to pos [W, 3]; rows: optional [W, >= nelec] float32 tensor
-        that receives the new orbital rows."""
+        that receives the new orbital rows.  Raises IndexError, without a
+        launch, when an earlier update is known to have been refused."""
         torch = _torch()
+        self.check_updates()
         W = int(pos.shape[0])
         dev = pos.device
         ratio = torch.empty(W, dtype=torch.float32, device=dev)
@@ -736,12 +751,14 @@ class Determinants:
         row k becomes rows[i] (rows: [W, >= nelec] float32 CUDA tensor).
         For a stream other than the current one, the matrices and rows have
         to be ready there, and accepted, if a tensor, on the current one.
-        An index out of range refuses the whole call on the GPU; the next
-        call raises IndexError for it."""
+        An index out of range raises IndexError at once where the host holds
+        the indices (a sequence, a tensor in host memory).  In a CUDA tensor
+        it refuses the whole call on the GPU, and check_updates, or the next
+        ratio or update after that, raises for it."""
         torch = _torch()
-        idx = self._index(accepted)
+        self.check_updates()
+        idx = self._index(accepted, min(len(self.A), len(self.ainv), len(rows)))
         n = int(idx.numel())
-        self._raise_refused()
         if n == 0:
             return
         if rows.device != self.A.device:
@@ -768,11 +785,15 @@ class Determinants:
                                                       _addr(self._status), _stream(torch, stream)):
             check()
 
-    def _raise_refused(self):
+    def check_updates(self):
+        """Raises IndexError, once, if an update whose launches are over (all
+        of them after a synchronisation) was refused for an index out of
+        range.  ratio and update begin with it; when it raises there, that
+        call has launched nothing and can be made again."""
         if self._refused is not None and self._refused.value:
             self._refused.value = 0
-            raise IndexError("Determinants.update: an earlier call's walker index was out of range; "
-                             "it updated nothing")
+            raise IndexError("Determinants: an earlier update's walker index was out of range and it updated "
+                             "nothing; no work was launched by this call")
 
     def __del__(self):
         # kept for the next object: a launch that refuses may still write it

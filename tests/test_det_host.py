@@ -41,3 +41,27 @@ def test_rows_of_another_device_are_refused(monkeypatch):
     with pytest.raises(RuntimeError):
         D.update(1, [0, 2], torch.empty((3, 4), device="meta"))
     assert not called
+
+
+@pytest.mark.parametrize("bad", [3, -4])
+@pytest.mark.parametrize("make", ["list", "int64", "int32"])
+def test_index_known_to_the_host_is_checked_at_once(monkeypatch, bad, make):
+    torch = pytest.importorskip("torch")
+    D, rows = population(torch)
+    launches = []
+
+    class Lib:
+        def einspline_gb300_det_update_accepted(self, *a):
+            launches.append(a)
+            return 0
+
+    monkeypatch.setattr(api, "_lib", Lib)
+    monkeypatch.setattr(api, "_stream", lambda torch, stream: 5)
+    as_given = lambda v: v if make == "list" else torch.tensor(v, dtype=getattr(torch, make))  # noqa: E731
+    with pytest.raises(IndexError):
+        D.update(1, as_given([0, bad, 1]), rows)
+    with pytest.raises(IndexError):
+        D.update(1, as_given([0, 2]), rows[:2])  # beyond the rows
+    assert not launches
+    D.update(1, as_given([0, -3, 2]), rows)
+    assert len(launches) == 1
