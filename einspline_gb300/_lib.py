@@ -229,6 +229,8 @@ def _signatures():
     sig["einspline_gb300_det_update"] = ([C.POINTER(DetOpts), i32, vp, vp, vp, vp, vp], i32)
     sig["einspline_gb300_det_update_accepted"] = ([C.POINTER(DetOpts), i32, vp, C.POINTER(DetBatch), vp, vp, vp, vp],
                                                   i32)
+    sig["einspline_gb300_det_update_accepted_mark"] = (
+        [C.POINTER(DetOpts), i32, vp, C.POINTER(DetBatch), vp, vp, vp, i32, vp], i32)
     sig["einspline_gb300_server_create"] = ([vp, C.POINTER(ServerOpts)], vp)
     sig["einspline_gb300_server_destroy"] = ([vp], i32)
     sig["einspline_gb300_server_submit"] = ([vp, vp, i32], i64)

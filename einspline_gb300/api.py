@@ -10,7 +10,9 @@ libeinspline_gb300.so; torch is used only to hold device buffers.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
+import itertools
 
 import numpy as np
 
@@ -671,14 +673,7 @@ class Determinants:
         self.W, self.ld = int(A.shape[0]), int(ainv.shape[-1])
         self.nelec, self.trans = int(nelec), int(trans)
         self._cache = {}
-        self._status = self._refused = None  # host tensors: nothing runs that could refuse
-        if A.is_cuda:
-            try:
-                self._status = _status_words.pop()
-            except IndexError:
-                self._status = torch.zeros(1, dtype=torch.int32).pin_memory()
-            self._refused = C.c_int.from_address(self._status.data_ptr())
-            self._refused.value = 0
+        self._status = _StatusWord() if A.is_cuda else None  # host tensors: nothing runs that could refuse
         self.a_ptrs = self._ptrs(A)
         self.ainv_ptrs = self._ptrs(ainv)
         self.work = torch.empty(2 * self.nelec * self.W, dtype=torch.float32, device=A.device)
@@ -780,9 +775,10 @@ class Determinants:
             self.work.record_stream(stream)
         at = lambda t: (t.data_ptr(), t.stride(0) * t.element_size(), t.shape[0])  # noqa: E731
         o, b = self.opts(k), L.DetBatch(*at(self.A), *at(self.ainv), *at(rows))
-        if _lib().einspline_gb300_det_update_accepted(C.byref(o), n, idx.data_ptr(), C.byref(b),
-                                                      self.work.data_ptr(), scratch.data_ptr(),
-                                                      _addr(self._status), _stream(torch, stream)):
+        status, mark = (self._status.address, self._status.mark) if self._status else (None, 1)
+        if _lib().einspline_gb300_det_update_accepted_mark(C.byref(o), n, idx.data_ptr(), C.byref(b),
+                                                           self.work.data_ptr(), scratch.data_ptr(), status, mark,
+                                                           _stream(torch, stream)):
             check()
 
     def check_updates(self):
@@ -790,18 +786,44 @@ class Determinants:
         of them after a synchronisation) was refused for an index out of
         range.  ratio and update begin with it; when it raises there, that
         call has launched nothing and can be made again."""
-        if self._refused is not None and self._refused.value:
-            self._refused.value = 0
+        if self._status and self._status.refused():
             raise IndexError("Determinants: an earlier update's walker index was out of range and it updated "
                              "nothing; no work was launched by this call")
 
+
+class _StatusWord:
+    """A word of pinned host memory in which the GPU leaves this object's mark
+    when it refuses an update.  Words go from objects that are gone to new
+    ones, and a launch of the former owner may still write its mark, so marks
+    are never used twice."""
+
+    _free = collections.deque()  # (word, address) of words without an owner
+    _marks = itertools.count(1)
+
+    def __init__(self):
+        try:
+            self._word, self.address = self._free.pop()
+        except IndexError:
+            page = _torch().zeros(64, dtype=_torch().int32).pin_memory()
+            words = [(page[i], page.data_ptr() + 4 * i) for i in range(64)]
+            self._word, self.address = words.pop()
+            self._free.extend(words)
+        self._value = C.c_int.from_address(self.address)
+        self.mark = next(self._marks)
+
+    def refused(self):
+        """Whether the GPU refused since the last time this was true."""
+        if self._value.value != self.mark:
+            return False
+        self._value.value = 0
+        return True
+
+    def __reduce__(self):  # a copy is another object
+        return _StatusWord, ()
+
     def __del__(self):
-        # kept for the next object: a launch that refuses may still write it
-        if getattr(self, "_status", None) is not None and _status_words is not None:
-            _status_words.append(self._status)
-
-
-_status_words = []  # pinned words of objects that are gone
+        if hasattr(self, "mark"):
+            self._free.append((self._word, self.address))
 
 
 def launch_count() -> int:

@@ -1008,7 +1008,7 @@ struct PickArgs {
   char *base[3];
   int64_t step[3], count[3];
   int64_t *out;  // [3][naccept], then the refusal
-  int *status;
+  int *status, mark;
   int naccept;
 };
 __global__ void __launch_bounds__(1024) k_det_pick(const PickArgs a) {
@@ -1026,7 +1026,9 @@ __global__ void __launch_bounds__(1024) k_det_pick(const PickArgs a) {
   if (threadIdx.x == 0) {
     a.out[3 * (int64_t)a.naccept] = bad;
     if (bad && a.status) {
-      *(volatile int *)a.status = 1;
+      // an earlier owner's late refusal (a smaller mark) leaves this one's
+      if (a.mark) atomicMax_system(a.status, a.mark);
+      else *(volatile int *)a.status = 1;
       __threadfence_system();
     }
   }
@@ -1308,10 +1310,9 @@ int einspline_gb300_det_update(const einspline_gb300_det_opts *o, int naccept, f
   return update_walkers(d, naccept, stream ? (cudaStream_t)stream : cudaStreamLegacy);
 }
 
-int einspline_gb300_det_update_accepted(const einspline_gb300_det_opts *o, int naccept, const int64_t *accepted_d,
-                                        const einspline_gb300_det_batch *b, float *work_d, int64_t *ptrs_d,
-                                        int *status, void *stream) {
-  static const char *fn = "einspline_gb300_det_update_accepted";
+static int update_accepted(const char *fn, const einspline_gb300_det_opts *o, int naccept, const int64_t *accepted_d,
+                           const einspline_gb300_det_batch *b, float *work_d, int64_t *ptrs_d, int *status, int mark,
+                           void *stream) {
   clear();
   if (int r = check_det_opts(o, fn)) return r;
   if (naccept < 0) return fail(EINSPLINE_GB300_EINVAL, "%s: naccept < 0", fn);
@@ -1327,6 +1328,7 @@ int einspline_gb300_det_update_accepted(const einspline_gb300_det_opts *o, int n
   p.count[0] = b->a_count; p.count[1] = b->ainv_count; p.count[2] = b->row_count;
   p.out = ptrs_d;
   p.status = status;
+  p.mark = mark;
   p.naccept = naccept;
   k_det_pick<<<1, naccept >= 1024 ? 1024 : (naccept + 31) / 32 * 32, 0, s>>>(p);
   EG_CUDA(cudaGetLastError());
@@ -1343,6 +1345,22 @@ int einspline_gb300_det_update_accepted(const einspline_gb300_det_opts *o, int n
   d.ld = o->ld;
   d.trans = o->ainv_trans;
   return update_walkers(d, naccept, s);
+}
+
+int einspline_gb300_det_update_accepted(const einspline_gb300_det_opts *o, int naccept, const int64_t *accepted_d,
+                                        const einspline_gb300_det_batch *b, float *work_d, int64_t *ptrs_d,
+                                        int *status, void *stream) {
+  return update_accepted("einspline_gb300_det_update_accepted", o, naccept, accepted_d, b, work_d, ptrs_d, status, 0,
+                         stream);
+}
+
+int einspline_gb300_det_update_accepted_mark(const einspline_gb300_det_opts *o, int naccept, const int64_t *accepted_d,
+                                             const einspline_gb300_det_batch *b, float *work_d, int64_t *ptrs_d,
+                                             int *status, int mark, void *stream) {
+  static const char *fn = "einspline_gb300_det_update_accepted_mark";
+  clear();
+  if (mark < 1) return fail(EINSPLINE_GB300_EINVAL, "%s: mark must be positive", fn);
+  return update_accepted(fn, o, naccept, accepted_d, b, work_d, ptrs_d, status, mark, stream);
 }
 
 }  // extern "C"

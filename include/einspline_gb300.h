@@ -391,6 +391,14 @@ typedef struct {
 int einspline_gb300_det_update_accepted(const einspline_gb300_det_opts *opts, int naccept, const int64_t *accepted_d,
                                         const einspline_gb300_det_batch *batch, float *work_d, int64_t *ptrs_d,
                                         int *status, void *stream);
+/* The same for a status word that passes from one owner to the next while
+ * launches of the former may still be pending: a refusal raises *status to
+ * mark (positive) and never lowers it, so that an owner with a mark larger
+ * than those before it finds its own mark there exactly when a call of its
+ * own was refused. */
+int einspline_gb300_det_update_accepted_mark(const einspline_gb300_det_opts *opts, int naccept,
+                                             const int64_t *accepted_d, const einspline_gb300_det_batch *batch,
+                                             float *work_d, int64_t *ptrs_d, int *status, int mark, void *stream);
 
 /* FP64 (d and z) tables: how evaluations compute.
  *   0 (default): IEEE FP64 fused multiply-adds.  On GB300 the FP64 pipe is a

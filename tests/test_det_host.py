@@ -22,7 +22,7 @@ def test_update_reaches_the_library(monkeypatch):
     D, rows = population(torch)
 
     class Lib:
-        def einspline_gb300_det_update_accepted(self, o, n, idx, batch, work, scratch, status, stream):
+        def einspline_gb300_det_update_accepted_mark(self, o, n, idx, batch, work, scratch, status, mark, stream):
             assert n == 2 and idx and work and scratch and not status and stream == 5
             return 0
 
@@ -51,7 +51,7 @@ def test_index_known_to_the_host_is_checked_at_once(monkeypatch, bad, make):
     launches = []
 
     class Lib:
-        def einspline_gb300_det_update_accepted(self, *a):
+        def einspline_gb300_det_update_accepted_mark(self, *a):
             launches.append(a)
             return 0
 
@@ -65,3 +65,32 @@ def test_index_known_to_the_host_is_checked_at_once(monkeypatch, bad, make):
     assert not launches
     D.update(1, as_given([0, -3, 2]), rows)
     assert len(launches) == 1
+
+
+def test_status_words_change_owners(monkeypatch):
+    """What the GPU may still write for a word's former owner is not read as
+    the new owner's, and does not hide the new owner's own refusal."""
+    import copy
+    import ctypes
+    torch = pytest.importorskip("torch")
+    monkeypatch.setattr(torch.Tensor, "pin_memory", lambda t: t)
+    monkeypatch.setattr(api._StatusWord, "_free", type(api._StatusWord._free)())
+
+    def refuse(address, mark):  # the kernel's atomicMax
+        w = ctypes.c_int.from_address(address)
+        w.value = max(w.value, mark)
+
+    words = [api._StatusWord() for _ in range(70)]
+    assert len({w.address for w in words}) == 70
+    address, mark = words[5].address, words[5].mark
+    words[5] = None
+    new = api._StatusWord()
+    assert new.address == address and new.mark > mark
+    refuse(address, mark)
+    assert not new.refused()
+    refuse(address, new.mark)
+    refuse(address, mark)
+    assert new.refused() and not new.refused()
+    refuse(address, new.mark)
+    other = copy.deepcopy(new)
+    assert other.address != address and not other.refused() and new.refused()

@@ -36,7 +36,7 @@ class Recorder:
 
     cuda_stream = 7
 
-    def einspline_gb300_det_update_accepted(self, o, n, idx, batch, work, scratch, status, stream):
+    def einspline_gb300_det_update_accepted_mark(self, o, n, idx, batch, work, scratch, status, mark, stream):
         self.log.append(("launch", idx, work, stream))
         return 0
 

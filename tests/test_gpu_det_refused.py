@@ -49,3 +49,31 @@ def test_check_updates_reports_once():
     torch.cuda.synchronize()
     D.check_updates()
     assert torch.equal(D.A[0, K], rows[0])
+
+
+@pytest.mark.gpu
+def test_a_late_refusal_is_not_the_next_objects():
+    """A launch that is still pending when its object goes, and is refused
+    then, says nothing about an object made since."""
+    torch = pytest.importorskip("torch")
+    big = torch.zeros(256 << 20, device="cuda")
+    bad, good = torch.tensor([W], device="cuda"), torch.tensor([0], device="cuda")
+    D, rows = population(torch)
+    D.update(K, good, rows)
+    torch.cuda.synchronize()
+    done = torch.cuda.Event()
+    for _ in range(100):
+        big.add_(1.0)  # tens of milliseconds in front of the refusal
+    D.update(K, bad, rows)
+    done.record()
+    del D
+    others = [population(torch)[0] for _ in range(3)]
+    assert not done.query()
+    torch.cuda.synchronize()
+    for E in others:
+        E.check_updates()
+    others[0].update(K, bad, rows)
+    torch.cuda.synchronize()
+    others[1].check_updates()
+    with pytest.raises(IndexError):
+        others[0].check_updates()
