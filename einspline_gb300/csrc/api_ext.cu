@@ -11,6 +11,7 @@
 #include <chrono>
 
 #include "eg_internal.h"
+#include "sort_slices.h"
 
 namespace eg {
 
@@ -80,26 +81,19 @@ __device__ __forceinline__ unsigned coarse_cell(const EvalArgs &a, int ax, float
   return (unsigned)(i < 0 ? 0 : (i > a.lim[ax] ? a.lim[ax] : i)) >> shift;
 }
 
-__device__ __forceinline__ void slice_of(int n, int b, int &lo, int &hi) {
-  const int chunk = (n + (int)gridDim.x - 1) / (int)gridDim.x;
-  lo = min(n, b * chunk);
-  hi = min(n, lo + chunk);
-}
-
 __global__ void __launch_bounds__(kSortThreads) k_sort_keys(const EvalArgs a, int shift, unsigned short *key,
                                                             unsigned *hist) {
   __shared__ unsigned count[kCoarseKeys];
   const int tid = threadIdx.x;
-  int lo, hi;
-  slice_of((int)a.npts, blockIdx.x, lo, hi);
+  const SortSlice sl = sort_slice(a.npts, blockIdx.x, gridDim.x);
   for (int k = tid; k < kCoarseKeys; k += kSortThreads) count[k] = 0;
   __syncthreads();
-  for (int p = lo + tid; p < hi; p += kSortThreads) {
+  for (int64_t p = sl.lo + tid; p < sl.hi; p += kSortThreads) {
     float x[3];
 #pragma unroll
     for (int ax = 0; ax < 3; ax++)
-      x[ax] = a.pos_f64 ? (float)reinterpret_cast<const double *>(a.pos)[3 * (int64_t)p + ax]
-                        : reinterpret_cast<const float *>(a.pos)[3 * (int64_t)p + ax];
+      x[ax] = a.pos_f64 ? (float)reinterpret_cast<const double *>(a.pos)[3 * p + ax]
+                        : reinterpret_cast<const float *>(a.pos)[3 * p + ax];
     const unsigned k = (spread4(coarse_cell(a, 0, x[0], shift)) << 2) |
                        (spread4(coarse_cell(a, 1, x[1], shift)) << 1) | spread4(coarse_cell(a, 2, x[2], shift));
     key[p] = (unsigned short)k;
@@ -155,9 +149,8 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_scatter(int n, const unsi
     run += tot[j];
   }
   __syncthreads();
-  int lo, hi;
-  slice_of(n, b, lo, hi);
-  for (int p = lo + tid; p < hi; p += kSortThreads) perm[atomicAdd(&count[key[p]], 1u)] = p;
+  const SortSlice sl = sort_slice(n, b, gridDim.x);
+  for (int64_t p = sl.lo + tid; p < sl.hi; p += kSortThreads) perm[atomicAdd(&count[key[p]], 1u)] = (int)p;
 }
 
 static int coarse_shift(const EvalArgs &a) {
