@@ -632,10 +632,13 @@ int einspline_gb300_set_tile(einspline_gb300_table *t, int tx, int ty, int pb) {
   return 0;
 }
 
+// The shapes below are those of a batch that fills the GPU many times.
+static constexpr int64_t kReportPoints = 1 << 20;
+
 int einspline_gb300_get_tile(einspline_gb300_table *t, int *tx, int *ty, int *pb) {
   clear();
   if (!table3_ok(t) || !tx || !ty || !pb) return fail(EINSPLINE_GB300_EINVAL, "bad argument");
-  pick_tile(t, true, 1, *tx, *ty, *pb);
+  pick_tile(t, true, kReportPoints, *tx, *ty, *pb);
   return 0;
 }
 
@@ -643,15 +646,15 @@ int einspline_gb300_get_launch_shape(einspline_gb300_table *t, int sorted, int v
                                      int *mode) {
   clear();
   if (!table3_ok(t) || !tx || !ty || !pb || !mode) return fail(EINSPLINE_GB300_EINVAL, "bad argument");
-  pick_tile(t, vgh != 0, 1, *tx, *ty, *pb, sorted != 0);
-  *mode = pick_mode(t, vgh != 0, sorted != 0);
+  pick_tile(t, vgh != 0, kReportPoints, *tx, *ty, *pb, sorted != 0);
+  *mode = pick_mode(t, vgh != 0, sorted != 0, kReportPoints);
   return 0;
 }
 
 int einspline_gb300_get_load_mode(einspline_gb300_table *t) {
   clear();
   if (!table3_ok(t)) return fail(EINSPLINE_GB300_EINVAL, "bad table handle");
-  return pick_mode(t, true);
+  return pick_mode(t, true, false, kReportPoints);
 }
 
 }  // extern "C"

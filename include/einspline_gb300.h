@@ -253,7 +253,11 @@ int einspline_gb300_autotune(einspline_gb300_table *t, int64_t npts, int vgh);
  * override both; get_tile and get_load_mode report the random-order one. */
 int einspline_gb300_autotune_sorted(einspline_gb300_table *t, int64_t npts, int vgh);
 /* The tile and load mode a launch takes (random order or cell-sorted, vgh
- * or value-only), after set_tile / set_load_mode, tuning and defaults. */
+ * or value-only), after set_tile / set_load_mode, tuning and defaults, for a
+ * batch of about a million points; so do get_tile and get_load_mode (random
+ * order, vgh).  Defaults depend on the batch: one that leaves SMs idle runs
+ * in smaller blocks, and FP32 vgh of fewer than 20,000 values, or in cell order
+ * with less sharing of rows, in mode 2. */
 int einspline_gb300_get_launch_shape(einspline_gb300_table *t, int sorted, int vgh, int *tx, int *ty, int *pb,
                                      int *mode);
 
