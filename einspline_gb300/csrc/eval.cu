@@ -1637,6 +1637,9 @@ void pick_tile(Table *t, bool vgh, int64_t npts, int &tx, int &ty, int &pb, bool
     if (shared || tx > 64) tx = shared ? 32 : 64;
     ty = shared ? 4 : 1;
     pb = shared ? 8 : (!sorted && t->table_bytes < kL2Table) ? 4 : 1;
+    // billions of points of a few columns: a grid holds 2^31 - 1 blocks
+    const int tiles = (need + tx - 1) / tx;
+    while (pb < 64 && npts / pb * tiles > (1 << 30)) pb *= 2;
     return;
   }
   if (tx > 256) tx = 256;
