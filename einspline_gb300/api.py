@@ -673,6 +673,7 @@ class Determinants:
         self.W, self.ld = int(A.shape[0]), int(ainv.shape[-1])
         self.nelec, self.trans = int(nelec), int(trans)
         self._cache = {}
+        self._device = A.device
         self._status = _StatusWord() if A.is_cuda else None  # host tensors: nothing runs that could refuse
         self.a_ptrs = self._ptrs(A)
         self.ainv_ptrs = self._ptrs(ainv)
@@ -696,27 +697,22 @@ class Determinants:
             return self._remember(key, base + t.data_ptr())
         return self._cache[key]
 
-    def _index(self, accepted, count):
-        """accepted as int64 on the matrices' device.  Indices that the host
-        holds are checked here: -count <= index < count."""
+    def _index(self, accepted):
+        """accepted as int64 on the matrices' device, and the least and the
+        largest index where the host holds them (else None)."""
         torch = _torch()
         if isinstance(accepted, torch.Tensor):
-            if accepted.device.type == "cpu" and accepted.numel():
+            ends = None
+            if not accepted.is_cuda and accepted.numel():
                 accepted = accepted.to(torch.int64)
-                self._in_range(int(accepted.min()), int(accepted.max()), count)
-            return accepted.to(device=self.A.device, dtype=torch.int64)
+                ends = int(accepted.min()), int(accepted.max())
+            return accepted.to(device=self._device, dtype=torch.int64), ends
         key = ("i", tuple(int(i) for i in accepted))
-        if key[1]:
-            self._in_range(min(key[1]), max(key[1]), count)
-        if key not in self._cache:
-            return self._remember(key, torch.as_tensor(key[1], dtype=torch.int64, device=self.A.device))
-        return self._cache[key]
-
-    @staticmethod
-    def _in_range(lo, hi, count):
-        if lo < -count or hi >= count:
-            raise IndexError(f"Determinants.update: walker index {lo if lo < -count else hi} is out of range for "
-                             f"{count} walkers")
+        found = self._cache.get(key)
+        if found is None:
+            idx = torch.as_tensor(key[1], dtype=torch.int64, device=self._device)
+            found = self._remember(key, (idx, (min(key[1]), max(key[1])) if key[1] else None))
+        return found
 
     def opts(self, k, pos_f64=False, rule=1):
         return L.DetOpts(self.nelec, int(k), self.ld, self.trans, int(pos_f64), int(rule))
@@ -727,7 +723,9 @@ class Determinants:
         that receives the new orbital rows.  Raises IndexError, without a
         launch, when an earlier update is known to have been refused."""
         torch = _torch()
-        self.check_updates()
+        st = self._status
+        if st is not None and st.value.value == st.mark:
+            self.check_updates()
         W = int(pos.shape[0])
         dev = pos.device
         ratio = torch.empty(W, dtype=torch.float32, device=dev)
@@ -751,33 +749,40 @@ class Determinants:
         it refuses the whole call on the GPU, and check_updates, or the next
         ratio or update after that, raises for it."""
         torch = _torch()
-        self.check_updates()
-        idx = self._index(accepted, min(len(self.A), len(self.ainv), len(rows)))
+        st = self._status
+        if st is not None and st.value.value == st.mark:
+            self.check_updates()
+        idx, ends = self._index(accepted)
         n = int(idx.numel())
         if n == 0:
             return
-        if rows.device != self.A.device:
-            raise RuntimeError(f"Determinants.update: rows are on {rows.device}, the matrices on {self.A.device}")
+        if rows.device != self._device:
+            raise RuntimeError(f"Determinants.update: rows are on {rows.device}, the matrices on {self._device}")
+        at = lambda t: (t.data_ptr(), t.stride(0) * t.element_size(), t.shape[0])  # noqa: E731
+        o, b = self.opts(k), L.DetBatch(*at(self.A), *at(self.ainv), *at(rows))
+        if ends is not None:
+            count = min(b.a_count, b.ainv_count, b.row_count)
+            if ends[0] < -count or ends[1] >= count:
+                raise IndexError(f"Determinants.update: walker index {ends[0] if ends[0] < -count else ends[1]} is out "
+                                 f"of range for {count} walkers")
         idx = idx.contiguous()
         if stream is not None and not isinstance(stream, torch.cuda.Stream):
             stream = torch.cuda.ExternalStream(stream.cuda_stream)  # another library's
-        if stream is None or stream == torch.cuda.current_stream(self.A.device):
-            scratch = torch.empty(3 * n + 1, dtype=torch.int64, device=self.A.device)
+        if stream is None or stream == torch.cuda.current_stream(self._device):
+            scratch = torch.empty(3 * n + 1, dtype=torch.int64, device=self._device)
         else:
             # the scratch is the stream's own memory, what the current stream
             # still does to the indices comes first, and the stream may go on
             # using them and the work space after they are dropped here
             if isinstance(accepted, torch.Tensor):
-                stream.wait_stream(torch.cuda.current_stream(self.A.device))
+                stream.wait_stream(torch.cuda.current_stream(self._device))
             with torch.cuda.stream(stream):
-                scratch = torch.empty(3 * n + 1, dtype=torch.int64, device=self.A.device)
+                scratch = torch.empty(3 * n + 1, dtype=torch.int64, device=self._device)
             idx.record_stream(stream)
             self.work.record_stream(stream)
-        at = lambda t: (t.data_ptr(), t.stride(0) * t.element_size(), t.shape[0])  # noqa: E731
-        o, b = self.opts(k), L.DetBatch(*at(self.A), *at(self.ainv), *at(rows))
-        status, mark = (self._status.address, self._status.mark) if self._status else (None, 1)
         if _lib().einspline_gb300_det_update_accepted_mark(C.byref(o), n, idx.data_ptr(), C.byref(b),
-                                                           self.work.data_ptr(), scratch.data_ptr(), status, mark,
+                                                           self.work.data_ptr(), scratch.data_ptr(),
+                                                           st and st.address, st.mark if st else 1,
                                                            _stream(torch, stream)):
             check()
 
@@ -786,7 +791,7 @@ class Determinants:
         of them after a synchronisation) was refused for an index out of
         range.  ratio and update begin with it; when it raises there, that
         call has launched nothing and can be made again."""
-        if self._status and self._status.refused():
+        if self._status is not None and self._status.refused():
             raise IndexError("Determinants: an earlier update's walker index was out of range and it updated "
                              "nothing; no work was launched by this call")
 
@@ -808,14 +813,14 @@ class _StatusWord:
             words = [(page[i], page.data_ptr() + 4 * i) for i in range(64)]
             self._word, self.address = words.pop()
             self._free.extend(words)
-        self._value = C.c_int.from_address(self.address)
+        self.value = C.c_int.from_address(self.address)
         self.mark = next(self._marks)
 
     def refused(self):
         """Whether the GPU refused since the last time this was true."""
-        if self._value.value != self.mark:
+        if self.value.value != self.mark:
             return False
-        self._value.value = 0
+        self.value.value = 0
         return True
 
     def __reduce__(self):  # a copy is another object

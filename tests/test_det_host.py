@@ -94,3 +94,10 @@ def test_status_words_change_owners(monkeypatch):
     refuse(address, new.mark)
     other = copy.deepcopy(new)
     assert other.address != address and not other.refused() and new.refused()
+
+
+def test_no_rows_are_needed_without_an_accepted_walker():
+    torch = pytest.importorskip("torch")
+    D, _ = population(torch)
+    assert D.update(1, [], None) is None
+    assert D.update(1, torch.zeros(0, dtype=torch.int64), None) is None
