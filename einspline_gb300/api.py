@@ -33,11 +33,13 @@ def _torch():
 
 
 def _stream(torch, stream):
-    """Handle of stream, or of the current device's current one (as
-    torch.cuda.current_stream gives it, without a Stream object per call)."""
+    """Handle of stream, or of the current device's current one.  The raw
+    handle spares a Stream object per call, where torch has that function
+    (it is not public)."""
     if stream is not None:
         return stream.cuda_stream
-    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(torch.cuda.current_device()) if raw is not None else torch.cuda.current_stream().cuda_stream
 
 
 def _addr(t):
