@@ -806,6 +806,7 @@ int einspline_gb300_autotune(einspline_gb300_table *t, int64_t npts, int vgh) {
   if (r) return r;
   const int v = vgh ? 1 : 0;
   t->tuned_tx[v] = shape[0]; t->tuned_ty[v] = shape[1]; t->tuned_pb[v] = shape[2]; t->tuned_mode[v] = shape[3];
+  t->tuned_n[v] = npts;
   return 0;
 }
 
@@ -840,6 +841,7 @@ int einspline_gb300_autotune_sorted(einspline_gb300_table *t, int64_t npts, int 
       const int v = vgh ? 1 : 0;
       t->tuned_s_tx[v] = shape[0]; t->tuned_s_ty[v] = shape[1]; t->tuned_s_pb[v] = shape[2];
       t->tuned_s_mode[v] = shape[3];
+      t->tuned_s_n[v] = npts;
     }
   }
   cudaFree(buf);

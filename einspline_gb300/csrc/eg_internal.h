@@ -169,6 +169,7 @@ struct einspline_gb300_table {
   int tuned_tx[2] = {0, 0}, tuned_ty[2] = {0, 0}, tuned_pb[2] = {0, 0}, tuned_mode[2] = {0, 0};
   // the same for launches that visit points in cell order (sorted batches)
   int tuned_s_tx[2] = {0, 0}, tuned_s_ty[2] = {0, 0}, tuned_s_pb[2] = {0, 0}, tuned_s_mode[2] = {0, 0};
+  int64_t tuned_n[2] = {0, 0}, tuned_s_n[2] = {0, 0};  // the points a call that each was tuned for
 };
 
 namespace eg {

@@ -1363,10 +1363,15 @@ static int num_sms() {
 //   300       18.2 / 13.9 / 13.6 10.8 / 9.3 / 8.8   27.5 / 8.0 / 8.0   18.8 / 6.6 / 6.6
 //   1000      53.1 / 53 / 51     29.0 / 29 / 29     31.6 / 18.9 / 18.9 18.9 / 14.7 / 14.5
 //   3000      unchanged          unchanged          52.1 / 45 / 44     34.4 / 32 / 32
-// A batch of at least one full wave keeps the shape, as do shapes set by
-// set_tile.
+// A batch of at least one full wave keeps the shape; so do shapes set by
+// set_tile, and tuned ones at about the count of points they were tuned for.
 void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) {
   if (t->tile_tx || a.npts <= 0) return;
+  // a tuned shape was the fastest for its count of points: it stays down to
+  // half of them (FP64 30^3 x 203 values, 1000 points: 51 us, refitted 60)
+  const int v = vgh ? 1 : 0;
+  const int64_t tuned = a.perm && t->tuned_s_tx[v] ? t->tuned_s_n[v] : t->tuned_tx[v] ? t->tuned_n[v] : 0;
+  if (tuned && 2 * a.npts >= tuned) return;
   if (a.npts == 1) {
     // what the search below finds, without its 0.3 us
     tx = 32;
