@@ -1439,6 +1439,16 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
     }
     return;
   }
+  // A block's start costs it `start` eighths of a round, and an SM is no faster
+  // with fewer threads than `latency`, in which one round's loads and
+  // arithmetic hide behind each other.  FP64 values: without these, 30^3 x 33
+  // columns, 3500 points ran in two one-warp blocks an SM, each of 12 points
+  // one after another: 85 us, 35 now; 17 columns 88 us, 23 now.
+  int start = 0, latency = 0;
+  if (deal && !vgh) {
+    start = 1;
+    latency = 256;
+  }
   // modes 3 and 5 have one block width; the others' blocks narrow by halves
   const bool fixed = b.mode == 3 || b.mode == 5;
   const int width = fixed ? tx : (int)block.x, lanes = (int)block.y;
@@ -1453,7 +1463,8 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
       for (int p = u; p <= pb; p += u) {
         const int64_t blocks = (a.npts + p - 1) / p * tiles, deep = (blocks + sms - 1) / sms;
         if (deep > fit) continue;
-        const int64_t chain = rounds(x, y, p), work = deep * chain * x * y;
+        const int64_t chain = rounds(x, y, p);
+        const int64_t work = std::max((8 * chain + start) * deep * x * y, 8 * chain * latency);
         if (work < best_work || (work == best_work && chain < best_chain)) {
           best_work = work;
           best_chain = chain;

@@ -1,0 +1,47 @@
+"""The launch shape picked for a batch is not slower than a fixed one, at
+sizes where the rules had picked badly (times on the GPU; each was at least
+1.1 times as long there)."""
+import pytest
+
+from einspline_gb300 import api
+
+
+def fastest(torch, f, runs=20):
+    for _ in range(5):
+        f()
+    best = float("inf")
+    for _ in range(runs):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(10):
+            f()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+CASES = [
+    # FP64 values of few columns: a block of one warp does one point at a time
+    ("d", api.STORE_NATIVE, 30, 17, 3500, False, False, (32, 8, 16)),
+    ("d", api.STORE_NATIVE, 30, 33, 3500, False, False, (32, 8, 15)),
+    ("d", api.STORE_NATIVE, 30, 33, 1500, False, False, (32, 8, 15)),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,storage,g,N,P,vgh,sort,shape", CASES)
+def test_picked_shape_is_not_slower(kind, storage, g, N, P, vgh, sort, shape):
+    torch = pytest.importorskip("torch")
+    dt = torch.float64 if kind == "d" else torch.float32
+    G = api.MultiUBspline3D(kind, [(0.0, 1.0, g)] * 3, [(api.PERIODIC, api.PERIODIC)] * 3, N, storage=storage)
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(7)
+    G.set_device(0, torch.rand((N, g, g, g), dtype=dt, device="cuda", generator=gen))
+    G.flush()
+    pos = torch.rand((P, 3), dtype=dt, device="cuda", generator=gen)
+    out = G.eval(pos, vgh=vgh)
+    run = lambda: G.eval(pos, vgh=vgh, sort=sort, out=out)  # noqa: E731
+    picked = fastest(torch, run)
+    G.set_tile(*shape)
+    assert picked < 1.08 * fastest(torch, run)
