@@ -1390,7 +1390,7 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   const int64_t per = wave / sms;
   if (per < 1) return;
   // points a block works on at once, and rounds it takes for p points
-  const int need = (t->ncol + elems_per_thread(t) - 1) / elems_per_thread(t);
+  const int VW = elems_per_thread(t), need = (t->ncol + VW - 1) / VW;
   const bool deal = b.mode == 0 && deals(kernel_storage(t));
   auto at_once = [&](int x, int y) { return deal ? std::min(pb, x * y / std::min(x, need)) : y; };
   auto rounds = [&](int x, int y, int p) { return deal ? (p * std::min(x, need) + x * y - 1) / (x * y) : p / y; };
@@ -1403,7 +1403,7 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   // groups' blocks; the wide value kernel deals the columns of a ragged last
   // tile to all its threads, so that tile counts by its share of the columns
   const bool dealt = b.mode == 3 && !vgh;
-  const int64_t tcols = (int64_t)tx * elems_per_thread(t) * 2;
+  const int64_t tcols = (int64_t)tx * VW * 2;
   auto blocks_of = [&](int64_t groups) { return dealt ? (groups * a.ncol + tcols - 1) / tcols : groups * b.ntiles; };
   const int64_t full = (a.npts + pb - 1) / pb * b.ntiles;
   if (full >= wave && deal) {
@@ -1443,11 +1443,18 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   // with fewer threads than `latency`, in which one round's loads and
   // arithmetic hide behind each other.  FP64 values: without these, 30^3 x 33
   // columns, 3500 points ran in two one-warp blocks an SM, each of 12 points
-  // one after another: 85 us, 35 now; 17 columns 88 us, 23 now.
+  // one after another: 85 us, 35 now; 17 columns 88 us, 23 now.  16-bit values,
+  // the FP32 vgh copy pipeline and the tensor cores, which had taken the
+  // shortest of equal chains: F16 64 x 60 x 56 x 203 values, 7000 points 45 ->
+  // 37, FP32 x 400 vgh, 1000 points 34.8 -> 30.5, F16 x 128 vgh, 2500 points
+  // 22.7 -> 18.4.
   int start = 0, latency = 0;
   if (deal && !vgh) {
     start = 1;
     latency = 256;
+  } else if (dealt || b.mode == 5 || (b.mode == 2 && kernel_storage(t) == ST_F32)) {
+    start = 1;
+    latency = 128;
   }
   // modes 3 and 5 have one block width; the others' blocks narrow by halves
   const bool fixed = b.mode == 3 || b.mode == 5;
@@ -1463,7 +1470,8 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
       for (int p = u; p <= pb; p += u) {
         const int64_t blocks = (a.npts + p - 1) / p * tiles, deep = (blocks + sms - 1) / sms;
         if (deep > fit) continue;
-        const int64_t chain = rounds(x, y, p);
+        // (a single dealt tile takes as many rounds as its pairs do)
+        const int64_t chain = dealt && b.ntiles == 1 ? (p * ((a.ncol + 2 * VW - 1) / (2 * VW)) + x - 1) / x : rounds(x, y, p);
         const int64_t work = std::max((8 * chain + start) * deep * x * y, 8 * chain * latency);
         if (work < best_work || (work == best_work && chain < best_chain)) {
           best_work = work;

@@ -26,6 +26,10 @@ CASES = [
     ("d", api.STORE_NATIVE, 30, 17, 3500, False, False, (32, 8, 16)),
     ("d", api.STORE_NATIVE, 30, 33, 3500, False, False, (32, 8, 15)),
     ("d", api.STORE_NATIVE, 30, 33, 1500, False, False, (32, 8, 15)),
+    # copy pipelines and tensor cores: more, shorter blocks of equal work
+    ("s", api.STORE_F16, 30, 203, 7000, False, False, (32, 1, 8)),
+    ("s", api.STORE_I16, 30, 203, 7000, False, False, (32, 1, 8)),
+    ("s", api.STORE_F16, 64, 128, 2500, True, False, (128, 1, 10)),
 ]
 
 
