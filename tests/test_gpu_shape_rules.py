@@ -30,6 +30,9 @@ CASES = [
     ("s", api.STORE_F16, 30, 203, 7000, False, False, (32, 1, 8)),
     ("s", api.STORE_I16, 30, 203, 7000, False, False, (32, 1, 8)),
     ("s", api.STORE_F16, 64, 128, 2500, True, False, (128, 1, 10)),
+    # values in cell order: one point a lane, whose rows its neighbours share
+    ("s", api.STORE_NATIVE, 30, 64, 15000, False, True, (32, 8, 16)),
+    ("s", api.STORE_NATIVE, 30, 5, 15000, False, True, (32, 8, 16)),
 ]
 
 
