@@ -1434,12 +1434,17 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
     return;
   }
   if (full >= wave) {
-    // between one and two waves of the copy pipelines' blocks: the size whose
-    // whole waves take the least points one after another (FP32 48^3 x 400,
-    // 3001 points vgl: 51.4 us with 5 points a block, 57.5 with 8)
-    if (b.mode < 2 || b.mode > 4 || full > 2 * wave) return;
+    // between one and two waves of the copy pipelines' blocks, or of the FP32
+    // vgh direct-load blocks: the size whose whole waves take the least points
+    // one after another (FP32 48^3 x 400, 3001 points vgl: 51.4 us with 5
+    // points a block, 57.5 with 8; direct loads, 30^3 x 777, 1500 points vgh: 51
+    // us with 6 points, 59 with 8)
+    const bool direct = b.mode == 0 && vgh && kernel_storage(t) == ST_F32;
+    if (!(b.mode >= 2 && b.mode <= 4) && !direct) return;
+    if (full > 2 * wave) return;
+    const int step = direct ? (int)block.y : 1;
     int64_t best = INT64_MAX;
-    for (int p = pb, p0 = pb; p >= (p0 + 1) / 2; p--) {
+    for (int p = pb, p0 = pb; p >= (p0 + 1) / 2; p -= step) {
       const int64_t cost = (blocks_of((a.npts + p - 1) / p) + wave - 1) / wave * p;
       if (cost < best) {
         best = cost;

@@ -33,6 +33,9 @@ CASES = [
     # values in cell order: one point a lane, whose rows its neighbours share
     ("s", api.STORE_NATIVE, 30, 64, 15000, False, True, (32, 8, 16)),
     ("s", api.STORE_NATIVE, 30, 5, 15000, False, True, (32, 8, 16)),
+    # FP32 vgh by direct loads, a little more than a wave of blocks
+    ("s", api.STORE_NATIVE, 30, 777, 1500, True, False, (32, 2, 6)),
+    ("s", api.STORE_NATIVE, 30, 400, 2500, True, False, (32, 2, 6)),
 ]
 
 
