@@ -274,7 +274,9 @@ class MultiUBspline3D:
 
     def eval(self, pos, vgh=True, rule=0, layout=0, sort=False, out=None, stream=None):
         """einspline_gb300_eval_3d on torch CUDA tensors.  pos: [P, 3]
-        float32/float64.  Returns (vals, grads, hess) torch tensors."""
+        float32/float64.  sort: True visits the points in cell order, False
+        leaves their order to the library, -1 says that they come in it.
+        Returns (vals, grads, hess) torch tensors."""
         torch = _torch()
         P = int(pos.shape[0])
         if out is None:

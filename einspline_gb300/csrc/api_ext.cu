@@ -418,10 +418,14 @@ static int eval_device(Table *t, const einspline_gb300_eval_opts *o, int64_t npt
   a.npts = npts;
   a.pos = pos_d;
   a.vals = v; a.grads = g; a.hess = h;
-  if (!o->sort || npts <= 1) return launch_eval_ordered(t, a, o->vgh != 0, s);
-  int *perm = nullptr;
-  if (int r = sort_points(t, a, o->vgh != 0, &perm, s)) return r;
-  a.perm = perm;
+  if (!o->sort || (o->sort > 0 && npts <= 1)) return launch_eval_ordered(t, a, o->vgh != 0, s);
+  if (o->sort < 0) {
+    a.in_order = 1;
+  } else {
+    int *perm = nullptr;
+    if (int r = sort_points(t, a, o->vgh != 0, &perm, s)) return r;
+    a.perm = perm;
+  }
   int tx, ty, pb;
   pick_tile(t, o->vgh != 0, npts, tx, ty, pb, true);
   fit_tile(t, a, o->vgh != 0, tx, ty, pb);

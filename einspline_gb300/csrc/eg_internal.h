@@ -258,6 +258,7 @@ struct EvalArgs {
   int test_skip;              // mode 4 test hook: s + 1 makes block 0 issue no copy for
                               // its stage s, so that stage's wait runs out (0: off)
   int box_bytes;              // mode 4: bytes of one box row (<= 256 stored reals)
+  int in_order;               // host only: the points come in cell order (perm may be null)
   // mode 4: the table as a 4D tensor [x][y][z][column] (column innermost);
   // CUtensorMap is 128-byte aligned, and so is EvalArgs
   CUtensorMap tmap;
@@ -284,7 +285,7 @@ int prepare_eval(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb, const 
 // sorted: the launch visits its points in cell order (a visiting order is
 // set), which has its own tuned shape.
 void pick_tile(Table *t, bool vgh, int64_t npts, int &tx, int &ty, int &pb, bool sorted = false);
-// Shrinks a picked tile for a batch (a.npts, a.perm) that would leave SMs idle.
+// Shrinks a picked tile for a batch (a.npts, its order) that would leave SMs idle.
 void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb);
 // Load mode of launches on this table (see EvalArgs::mode).
 int pick_mode(Table *t, bool vgh, bool sorted = false, int64_t npts = 1);

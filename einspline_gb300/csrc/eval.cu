@@ -1245,7 +1245,7 @@ static int shape_kernel(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb,
   if (tx < 32 || tx % 32 || ty < 1 || tx * ty > 256 || pb < 1 || pb > 64)
     return fail(EINSPLINE_GB300_EINVAL, "bad launch shape tx=%d ty=%d pb=%d", tx, ty, pb);
   a.pb = pb;
-  a.mode = mode >= 0 ? mode : pick_mode(t, vgh, a.perm != nullptr, a.npts);
+  a.mode = mode >= 0 ? mode : pick_mode(t, vgh, a.perm || a.in_order, a.npts);
   const int ks = kernel_storage(t);
   if (a.mode >= 2 && ks == ST_F64) a.mode = 0;        // IEEE FP64 is FMA-bound: no pipeline variant
   // tensor cores: F16 and BF16 tables; one column a thread, so not the
@@ -1370,7 +1370,8 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   // a tuned shape was the fastest for its count of points: it stays down to
   // half of them (FP64 30^3 x 203 values, 1000 points: 51 us, refitted 60)
   const int v = vgh ? 1 : 0;
-  const int64_t tuned = a.perm && t->tuned_s_tx[v] ? t->tuned_s_n[v] : t->tuned_tx[v] ? t->tuned_n[v] : 0;
+  const bool sorted = a.perm || a.in_order;
+  const int64_t tuned = sorted && t->tuned_s_tx[v] ? t->tuned_s_n[v] : t->tuned_tx[v] ? t->tuned_n[v] : 0;
   if (tuned && 2 * a.npts >= tuned) return;
   if (a.npts == 1) {
     // what the search below finds, without its 0.3 us
@@ -1405,7 +1406,7 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   const bool f64 = t->storage == ST_F64;
   if (b.mode == 0 && (f64 || !vgh)) {
     const int64_t blocks = (a.npts + pb - 1) / pb * b.ntiles;
-    const bool shared = !f64 && a.perm;
+    const bool shared = !f64 && sorted;
     if (shared && 2 * blocks >= wave) return;
     if (shared || blocks < (f64 ? 1 : 4) * wave) pb = at_once((int)block.x, (int)block.y);
   }

@@ -136,9 +136,13 @@ typedef struct {
                      table on different streams must not overlap.
                      0: the library decides: large batches on tables above
                      192 MB go in cell order too, in scratch made with the
-                     table (7 MB) and from any number of streams at once;
+                     table (5 MB) and from any number of streams at once;
                      others, and launches under stream capture, keep
-                     their order.  The *_cuda entries do the same          */
+                     their order.  The *_cuda entries do the same.
+                     -1: the points are taken to be in cell order already
+                     (any order is evaluated correctly): theirs is kept, and
+                     the launch has the shape for such batches, without the
+                     10-25 us that the ordering takes                      */
   int64_t vstride, gstride, hstride; /* per-point output strides in output
                      reals (float for s/c, double for d/z); 0 = packed       */
 } einspline_gb300_eval_opts;
