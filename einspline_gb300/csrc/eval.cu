@@ -87,7 +87,7 @@ __device__ __forceinline__ void st_shifted(float *p, const float (&v)[N], const 
 // real was a store of its own and a warp's store touched 32 sectors; one() is
 // that store, still taken by the lane at the table's ragged end.
 // 24,000 points, vgh: I16 48^3 x 777: 735 -> 529 us; FP32 45^3 x 203: 168 ->
-// 156, in the CPU layout 242 -> 169.
+// 154, in the CPU layout 242 -> 167.
 template <int N, typename One>
 __device__ __forceinline__ void st_run(float *p, const float (&v)[N], bool full, const LaneRuns &w, One one) {
   const unsigned off = (unsigned)reinterpret_cast<uintptr_t>(p) & 15u;
@@ -289,7 +289,7 @@ __device__ __forceinline__ void epilogue(const EvalArgs &a, int64_t src, int col
 // points are dealt to all threads in turn.  I16 56 x 60 x 52 x 777, 24,000
 // points: 264 -> 235 us (7 of these by decode2).  FP64, whose pipe takes
 // as long for an idle lane: complex 32 x 9 x 23 x 8, 12,392 points vgh: 527 ->
-// 161 us; 40^3 x 203 real, 8000 points: 1142 -> 994, values 332 -> 297.  The other kernels
+// 161 us; 40^3 x 203 real, 8000 points: 1204 -> 994, values 332 -> 297.  The other kernels
 // do not deal: their tiles are narrower, or in vgh a block-wide point index is
 // worth the 2-5 % that a thread's own costs.
 struct ColumnWalk {
@@ -1351,18 +1351,19 @@ static int num_sms() {
 // ones.  A block goes through its points one after another, so a batch of
 // 48 points in blocks of 8 or 10 left most SMs idle for 8 or 10 points'
 // time.  Among the shapes whose blocks are all resident at once, the one with
-// the least work on the fullest SM (points x columns), then the shortest
-// chain of points in a block; shapes with the same columns a block before
-// narrower ones.  Results do not depend on the shape.
+// the least work on the fullest SM (points x columns, with what a block's
+// start and too few threads cost), then the shortest chain of points in a
+// block; shapes with the same columns a block before narrower ones.  Results
+// do not depend on the shape.
 //
-// Measured, kernel time in us, given shape / this rule's / best of a scan
-// (vgh):
+// Measured, us a launch in a replayed graph, given shape / this rule's / best
+// of a scan (vgh):
 //             F32 64^3 x 1024    F16 64^3 x 1024    I16 64^3 x 512     F32 45^3 x 203
-//   8 points  17.1 / 3.8 / 3.8    9.1 / 4.1 / 4.1   27.1 / 5.3 / 5.3   18.5 / 3.9 / 3.9
-//   48        17.4 / 5.0 / 5.0   10.6 / 5.3 / 4.9   27.2 / 5.4 / 5.4   18.5 / 4.0 / 4.0
-//   300       18.2 / 13.9 / 13.6 10.8 / 9.3 / 8.8   27.5 / 8.0 / 8.0   18.8 / 6.6 / 6.6
-//   1000      53.1 / 53 / 51     29.0 / 29 / 29     31.6 / 18.9 / 18.9 18.9 / 14.7 / 14.5
-//   3000      unchanged          unchanged          52.1 / 45 / 44     34.4 / 32 / 32
+//   8 points  16.9 / 4.2 / 3.7    9.0 / 4.1 / 4.0   27.5 / 5.4 / 5.4   20.4 / 4.5 / 4.2
+//   48        17.2 / 4.9 / 4.9   10.5 / 4.8 / 4.8   27.4 / 5.5 / 5.5   20.4 / 4.6 / 4.3
+//   300       18.1 / 14.0 / 13.6 10.6 / 9.3 / 8.7   27.8 / 7.9 / 7.9   12.4 / 5.1 / 5.1
+//   1000      52.5 / 50.9 / 47.4 28.6 / 28.8 / 28.6 31.0 / 19.1 / 19.1 13.4 / 9.2 / 9.2
+//   3000      unchanged          unchanged          52.5 / 41.1 / 41.2 24.9 / 24.8 / 24.4
 // A batch of at least one full wave keeps the shape; so do shapes set by
 // set_tile, and tuned ones at about the count of points they were tuned for.
 void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) {
@@ -1572,11 +1573,6 @@ int prepare_eval(Table *t, EvalArgs &a, bool vgh, int tx, int ty, int pb, const 
   return 0;
 }
 
-// Untuned defaults for vgh are the autotuner's choices on GB300 at 64^3 x
-// 1024 and 128^3 x 2048 (and 48^3 x 512 double-float): the shared-memory
-// copy pipeline, 8-column wide for 16-bit tables; value-only evaluation uses
-// the wide pipeline for 16-bit tables and direct loads otherwise; IEEE FP64
-// (FMA-bound) always uses direct loads.
 // Points per stencil row that npts uniform points touch.
 static double row_reuse(const Table *t, int64_t npts) {
   const double R = (double)t->Nc[0] * t->Nc[1] * t->Nc[2], n64 = 64.0 * (double)std::max<int64_t>(npts, 1);
@@ -1607,6 +1603,12 @@ static bool direct_pays(const Table *t, bool sorted, int64_t npts) {
   return sorted && (t->table_bytes < kNearL2Table || row_reuse(t, npts) >= 3.0);
 }
 
+// Untuned defaults for vgh: the shared-memory copy pipeline, 8-column wide for
+// I16 tables (the autotuner's choices on GB300 at 64^3 x 1024 and 128^3 x 2048,
+// and 48^3 x 512 double-float), direct loads for FP32 tables where direct_pays,
+// the tensor cores for F16 and BF16; value-only evaluation uses the wide
+// pipeline for 16-bit tables and direct loads otherwise; IEEE FP64
+// (FMA-bound) always uses direct loads.
 int pick_mode(Table *t, bool vgh, bool sorted, int64_t npts) {
   if (t->tile_mode >= 0) return t->tile_mode;
   const int v = vgh ? 1 : 0;

