@@ -1457,7 +1457,8 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   }
   // A block's start costs it `start` eighths of a round, and an SM is no faster
   // with fewer threads than `latency`, in which one round's loads and
-  // arithmetic hide behind each other.  FP64 values: without these, 30^3 x 33
+  // arithmetic hide behind each other (of shapes that are below it, the one
+  // with the least on an SM).  FP64 values: without these, 30^3 x 33
   // columns, 3500 points ran in two one-warp blocks an SM, each of 12 points
   // one after another: 85 us, 35 now; 17 columns 88 us, 23 now.  16-bit values,
   // the FP32 vgh copy pipeline and the tensor cores, which had taken the
@@ -1476,7 +1477,7 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   const bool fixed = b.mode == 3 || b.mode == 5;
   const int width = fixed ? tx : (int)block.x, lanes = (int)block.y;
   int best[3] = {tx, ty, pb};
-  int64_t best_work = INT64_MAX, best_chain = 0;
+  int64_t best_work = INT64_MAX, best_load = 0, best_chain = 0;
   for (int x = width; x >= 32; x = x > 32 ? (x / 2 + 31) / 32 * 32 : 0) {
     if (fixed && x != width) break;
     const int64_t tiles = fixed ? b.ntiles : ((int64_t)b.ntiles * width + x - 1) / x;
@@ -1488,9 +1489,10 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
         if (deep > fit) continue;
         // (a single dealt tile takes as many rounds as its pairs do)
         const int64_t chain = dealt && b.ntiles == 1 ? (p * ((a.ncol + 2 * VW - 1) / (2 * VW)) + x - 1) / x : rounds(x, y, p);
-        const int64_t work = std::max((8 * chain + start) * deep * x * y, 8 * chain * latency);
-        if (work < best_work || (work == best_work && chain < best_chain)) {
+        const int64_t load = (8 * chain + start) * deep * x * y, work = std::max(load, 8 * chain * latency);
+        if (std::tie(work, load, chain) < std::tie(best_work, best_load, best_chain)) {
           best_work = work;
+          best_load = load;
           best_chain = chain;
           best[0] = x; best[1] = y; best[2] = p;
         }

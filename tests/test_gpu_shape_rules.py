@@ -26,6 +26,8 @@ CASES = [
     ("d", api.STORE_NATIVE, 30, 17, 3500, False, False, (32, 8, 16)),
     ("d", api.STORE_NATIVE, 30, 33, 3500, False, False, (32, 8, 15)),
     ("d", api.STORE_NATIVE, 30, 33, 1500, False, False, (32, 8, 15)),
+    # a few points: spread over the SMs, not in whole blocks on some
+    ("d", api.STORE_NATIVE, 30, 362, 31, False, False, (64, 1, 1)),
     # copy pipelines and tensor cores: more, shorter blocks of equal work
     ("s", api.STORE_F16, 30, 203, 7000, False, False, (32, 1, 8)),
     ("s", api.STORE_I16, 30, 203, 7000, False, False, (32, 1, 8)),
