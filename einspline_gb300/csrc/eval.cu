@@ -1455,24 +1455,28 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
     }
     return;
   }
-  // A block's start costs it `start` eighths of a round, and an SM is no faster
-  // with fewer threads than `latency`, in which one round's loads and
+  // A block's start costs as much as `start` threads' round, and an SM is no
+  // faster with fewer threads than `latency`, in which one round's loads and
   // arithmetic hide behind each other (of shapes that are below it, the one
-  // with the least on an SM).  FP64 values: without these, 30^3 x 33
-  // columns, 3500 points ran in two one-warp blocks an SM, each of 12 points
-  // one after another: 85 us, 35 now; 17 columns 88 us, 23 now.  16-bit values,
-  // the FP32 vgh copy pipeline and the tensor cores, which had taken the
-  // shortest of equal chains: F16 64 x 60 x 56 x 203 values, 7000 points 45 ->
-  // 37, FP32 x 400 vgh, 1000 points 34.8 -> 30.5, F16 x 128 vgh, 2500 points
-  // 22.7 -> 18.4.
+  // with the shortest chain, then the least on an SM).  FP64 values: without these, 30^3 x 33 columns,
+  // 3500 points ran in two one-warp blocks an SM, each of 12 points one after
+  // another: 85 us, 35 now; 17 columns 88 us, 23 now.  16-bit values, the FP32
+  // vgh copy pipeline and the tensor cores, which had taken the shortest of
+  // equal chains: F16 64 x 60 x 56 x 203 values, 7000 points 45 -> 37, FP32 x 400
+  // vgh, 1000 points 34.8 -> 30.5, F16 x 128 vgh, 2500 points 22.7 -> 18.4.
   int start = 0, latency = 0;
   if (deal && !vgh) {
-    start = 1;
+    start = 4;
     latency = 256;
-  } else if (dealt || b.mode == 5 || (b.mode == 2 && kernel_storage(t) == ST_F32)) {
-    start = 1;
+  } else if (b.mode == 5) {
+    start = 96;
+    latency = 192;
+  } else if (dealt || (b.mode == 2 && kernel_storage(t) == ST_F32)) {
+    start = 4;
     latency = 128;
   }
+  // threads of a block that work: the pipeline's are idle past the columns
+  auto busy = [&](int x, int y) { return b.mode == 2 && latency ? std::min(x, need) * y : x * y; };
   // modes 3 and 5 have one block width; the others' blocks narrow by halves
   const bool fixed = b.mode == 3 || b.mode == 5;
   const int width = fixed ? tx : (int)block.x, lanes = (int)block.y;
@@ -1487,10 +1491,11 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
       for (int p = u; p <= pb; p += u) {
         const int64_t blocks = (a.npts + p - 1) / p * tiles, deep = (blocks + sms - 1) / sms;
         if (deep > fit) continue;
-        // (a single dealt tile takes as many rounds as its pairs do)
-        const int64_t chain = dealt && b.ntiles == 1 ? (p * ((a.ncol + 2 * VW - 1) / (2 * VW)) + x - 1) / x : rounds(x, y, p);
-        const int64_t load = (8 * chain + start) * deep * x * y, work = std::max(load, 8 * chain * latency);
-        if (std::tie(work, load, chain) < std::tie(best_work, best_load, best_chain)) {
+        const int64_t chain = rounds(x, y, p), load = deep * (chain * busy(x, y) + start);
+        // a single dealt tile takes as many rounds as its pairs do
+        const int64_t turns = dealt && b.ntiles == 1 ? (p * ((a.ncol + 2 * VW - 1) / (2 * VW)) + x - 1) / x : chain;
+        const int64_t work = std::max(deep * (turns * busy(x, y) + start), turns * latency);
+        if (std::tie(work, chain, load) < std::tie(best_work, best_chain, best_load)) {
           best_work = work;
           best_load = load;
           best_chain = chain;
