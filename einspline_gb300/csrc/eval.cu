@@ -1359,11 +1359,11 @@ static int num_sms() {
 // Measured, us a launch in a replayed graph, given shape / this rule's / best
 // of a scan (vgh):
 //             F32 64^3 x 1024    F16 64^3 x 1024    I16 64^3 x 512     F32 45^3 x 203
-//   8 points  16.9 / 4.2 / 3.7    9.0 / 4.1 / 4.0   27.5 / 5.4 / 5.4   20.4 / 4.5 / 4.2
-//   48        17.2 / 4.9 / 4.9   10.5 / 4.8 / 4.8   27.4 / 5.5 / 5.5   20.4 / 4.6 / 4.3
-//   300       18.1 / 14.0 / 13.6 10.6 / 9.3 / 8.7   27.8 / 7.9 / 7.9   12.4 / 5.1 / 5.1
-//   1000      52.5 / 50.9 / 47.4 28.6 / 28.8 / 28.6 31.0 / 19.1 / 19.1 13.4 / 9.2 / 9.2
-//   3000      unchanged          unchanged          52.5 / 41.1 / 41.2 24.9 / 24.8 / 24.4
+//   8 points  16.8 / 3.7 / 3.6    8.9 / 4.1 / 4.0   27.2 / 5.4 / 5.4   20.2 / 4.2 / 4.2
+//   48        17.2 / 4.9 / 4.9   10.4 / 4.8 / 4.8   27.3 / 5.4 / 5.4   20.3 / 4.3 / 4.2
+//   300       18.1 / 14.0 / 13.9 10.6 / 8.7 / 8.7   27.8 / 7.9 / 7.9   12.3 / 5.1 / 5.1
+//   1000      52.7 / 47.5 / 47.6 28.7 / 28.8 / 28.7 31.0 / 19.3 / 19.1 13.3 / 9.2 / 9.3
+//   3000      unchanged          unchanged          52.6 / 41.2 / 41.1 24.8 / 24.7 / 24.4
 // A batch of at least one full wave keeps the shape; so do shapes set by
 // set_tile, and tuned ones at about the count of points they were tuned for.
 void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) {
@@ -1460,7 +1460,7 @@ void fit_tile(Table *t, const EvalArgs &a, bool vgh, int &tx, int &ty, int &pb) 
   // arithmetic hide behind each other (of shapes that are below it, the one
   // with the shortest chain, then the least on an SM).  FP64 values: without these, 30^3 x 33 columns,
   // 3500 points ran in two one-warp blocks an SM, each of 12 points one after
-  // another: 85 us, 35 now; 17 columns 88 us, 23 now.  16-bit values, the FP32
+  // another: 85 us, 33 now; 17 columns 88 us, 23 now.  16-bit values, the FP32
   // vgh copy pipeline and the tensor cores, which had taken the shortest of
   // equal chains: F16 64 x 60 x 56 x 203 values, 7000 points 45 -> 37, FP32 x 400
   // vgh, 1000 points 34.8 -> 30.5, F16 x 128 vgh, 2500 points 22.7 -> 18.4.
